@@ -13,29 +13,17 @@
 // cannot use mncclEmuCreate / mncclEmuCollective, which cudaMalloc the control
 // segments, inboxes and the parameter table.
 //
-// What it does: the same one-shot kernel (push into per-source inboxes, one
-// barrier per block, every virtual rank reduces all contributions in rank
-// order), launched once, cooperatively, over all virtual ranks.  The scratch it
-// needs (barrier words, per-rank state, inboxes) sits in a file-scope
-// `static __device__` array inside the library, kNoAllocScratchBytes large,
-// which every GPU that loads the library holds until the process exits.  The
-// kernel parameters travel by value.  No cudaMalloc, cudaFree or allocating
-// library routine is called, in set-up or later.
+// What it does: one kernel that reads every buffer, reduces in buffer order (fp32 accumulation for the
+// floating types, the bits of the one-shot collective kernel) and writes every result.  Pointers travel by
+// value; no cudaMalloc, cudaFree or allocating library routine is called, in set-up or later, and no
+// state is kept between calls except the two words of the outcome record, a `static __device__` array.
 //
 // Limits (requests beyond them are rejected with ncclInvalidArgument and a
 // message): 2..kNoAllocMaxRanks buffers, at most kNoAllocMaxBytes bytes each;
 // types fp32, fp16, bf16, int32; operators sum, prod, max, min, avg.
 //
-// First call on a device: looks up the device address of the scratch array
-// (cudaGetSymbolAddress, with that device current) and keeps it; make that
-// first call outside of any stream capture.
-//
-// Sharing: every call on a device uses the same array.  Each call first clears
-// the barrier words and per-rank state on `stream`, so it does not depend on
-// what the previous call left behind (a call that was aborted, say); the
-// inboxes are not cleared, they are always written before they are read.  Two
-// calls that overlap on the GPU (different streams, no ordering between them)
-// race on the array; order them.
+// send[r] may equal recv[r'] for any r, r'; buffers that overlap otherwise race.  Calls on different
+// streams do not disturb one another.
 #pragma once
 #include <stddef.h>
 
@@ -53,14 +41,12 @@ enum { kNoAllocMaxBytes = 64 * 1024 };
 ncclResult_t mncclLocalAllReduceNoAlloc(const void* const* send, void* const* recv, int nbuffers, size_t count,
                                         ncclDataType_t datatype, ncclRedOp_t op, cudaStream_t stream);
 
-/* Size in bytes of the static scratch array (per GPU). */
+/* Size in bytes of the static device memory (per GPU): the outcome record. */
 size_t mncclNoAllocScratchBytes(void);
 
-/* Outcome of the last call on the current device: *status 0 when every wait inside its kernel completed,
- * 1 when one ran out of its two-second budget, 2 when it was aborted; *detail (may be NULL) names the
- * block and the virtual rank that was waited for.  A call whose kernel gave up returns ncclSuccess all
- * the same and leaves its output incomplete, so a caller that cannot tolerate that asks here.
- * Synchronises `stream`, reads a few bytes of the scratch, allocates nothing. */
+/* Outcome of the last call on the current device: *status 0 (and *detail 0, may be NULL) when its kernel
+ * completed.  The kernel waits for nothing, so a call that was launched has no other outcome; the entry point
+ * stays for callers of earlier versions.  Synchronises `stream`, reads eight bytes, allocates nothing. */
 ncclResult_t mncclNoAllocLastStatus(cudaStream_t stream, unsigned* status, unsigned* detail);
 
 #ifdef __cplusplus
