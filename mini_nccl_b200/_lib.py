@@ -181,6 +181,29 @@ def lib() -> C.CDLL:
     return L
 
 
+_EXT = None
+
+
+def ext():
+    """The PyTorch extension behind the frequent calls (csrc/torch/ext.cpp), bound to the library that
+    :func:`lib` has loaded.  Built on first use if its file is missing."""
+    global _EXT
+    if _EXT is not None:
+        return _EXT
+    import torch  # noqa: F401  (its shared libraries must be in the process first)
+
+    L = lib()
+    if not (_HERE / "_torch_ext.so").exists():
+        from . import build as _build
+        _build.build_torch_ext()
+    from . import _torch_ext
+
+    address = lambda name: C.cast(getattr(L, name), C.c_void_p).value if hasattr(L, name) else 0
+    _torch_ext.bind(address("mncclAllReduceEx"), address("mncclCommGetAsyncError"), address("mncclGemmBf16"))
+    _EXT = _torch_ext
+    return _EXT
+
+
 def hooks_lib() -> C.CDLL:
     """The test-suite's own copy of the library (libmini_nccl_testhooks.so): the same objects plus the
     entry points of csrc/testing/hooks.cc.  It has its own static state, so a test that needs a hook to

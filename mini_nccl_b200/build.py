@@ -113,6 +113,33 @@ def lib_path() -> Path:
     return LIBDIR / "libmini_nccl.so"
 
 
+def build_torch_ext(verbose: bool = False) -> Path | None:
+    """The CPython extension behind the binding's frequent calls (csrc/torch/ext.cpp), compiled against the
+    installed PyTorch; None where there is none (the ctypes binding itself does not need it)."""
+    import importlib.util
+    import sysconfig
+
+    spec = importlib.util.find_spec("torch")
+    if spec is None or not spec.submodule_search_locations:
+        return None
+    torch_dir = Path(spec.submodule_search_locations[0])
+    out = ROOT / "mini_nccl_b200" / "_torch_ext.so"
+    src = CSRC / "torch" / "ext.cpp"
+    newest = max(src.stat().st_mtime, *(h.stat().st_mtime for h in (ROOT / "include").glob("*.h")))
+    if out.exists() and out.stat().st_mtime >= newest:
+        return out
+    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", "-shared", *_common_includes(),
+           "-isystem", str(torch_dir / "include"), "-isystem", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"),
+           "-I", sysconfig.get_paths()["include"], str(src), "-o", str(out), "-L", str(torch_dir / "lib"),
+           "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"build of the PyTorch extension failed\n{r.stderr}")
+    return out
+
+
 def build(verbose: bool = False, programs: bool = True, jobs: int | None = None) -> Path:
     """Build the shared library (and the programs).  Returns the library path."""
     if not Path(NVCC).exists():
@@ -156,6 +183,7 @@ def build(verbose: bool = False, programs: bool = True, jobs: int | None = None)
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link of the test hooks failed\n{r.stdout}\n{r.stderr}")
+    build_torch_ext(verbose)
     if programs:
         for name, (sources, needs_cuda) in PROGRAMS.items():
             paths = [ROOT / s for s in sources]

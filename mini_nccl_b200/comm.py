@@ -59,6 +59,7 @@ class Communicator:
         check(lib().mncclCommUserRank(self._h, C.byref(r)), "mncclCommUserRank")
         check(lib().mncclCommCount(self._h, C.byref(n)), "mncclCommCount")
         self.rank, self.size = r.value, n.value
+        self._all_reduce = _lib.ext().all_reduce if torch is not None else None
 
     @classmethod
     def from_env(cls) -> "Communicator":
@@ -101,17 +102,10 @@ class Communicator:
         ``out`` may have another floating dtype than ``tensor`` and ``wire_dtype`` may name the
         type the data crosses NVLink in (fp32 -> bf16 -> fp32 and the like); accumulation is
         always fp32."""
-        out = tensor if out is None else out
-        if not tensor.is_contiguous() or not out.is_contiguous():
-            raise ValueError("all_reduce needs contiguous tensors")
-        if out.numel() != tensor.numel():
-            raise ValueError("size mismatch")
-        st = _torch_dtype_code(tensor.dtype)
-        rt = _torch_dtype_code(out.dtype)
-        wt = _torch_dtype_code(wire_dtype) if wire_dtype is not None else (rt if st == rt else _lib.BFLOAT16)
-        check(lib().mncclAllReduceEx(tensor.data_ptr(), st, out.data_ptr(), rt, wt, tensor.numel(), _OPS[op],
-                                     float(scale), _ALGOS[algo], self._h, self._stream_ptr(stream)), "mncclAllReduceEx")
-        return out
+        code = self._all_reduce(self._h.value or 0, tensor, out, wire_dtype, _OPS[op], scale, _ALGOS[algo], stream)
+        if code != _lib.SUCCESS:
+            raise MiniNcclError(code, "mncclAllReduceEx")
+        return tensor if out is None else out
 
     def reduce_scatter(self, tensor, out, op: str = "sum", stream=None):
         if tensor.numel() != out.numel() * self.size:
