@@ -14,14 +14,14 @@ bool nvls_type_ok(DType in, DType wire, DType out, RedOp op) {
                                     (in == DType::Bfloat16 && out == DType::Float32));
 }
 
+uint64_t ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
+
+}  // namespace
+
 bool triple_ok(DType in, DType wire, DType out, RedOp op) {
   if (in == wire && wire == out) return true;
   return nvls_type_ok(in, wire, out, op);  // the mixed triples are the same set
 }
-
-uint64_t ceil_div(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
-
-}  // namespace
 
 Algo parse_algo(const std::string& s) {
   const char* c = s.c_str();
@@ -90,9 +90,7 @@ Plan make_plan(const PlanInput& in, const CommCaps& caps, const Config& cfg) {
 
   if (N == 1) {
     if (in.mode != Mode::AllReduce && in.in != in.out) { p.reason = "type conversion needs AllReduce"; return p; }
-    p.spec.algo = Algo::Local;
-    const uint64_t vecs = ceil_div(in.count, std::min<uint64_t>(16 / dtype_size(in.in), 16 / osz));
-    p.spec.nblocks = static_cast<int>(std::clamp<uint64_t>(ceil_div(vecs, 512 * 4), 1, caps.sm_count * 4));
+    p.spec.algo = Algo::Local;   // no collective kernel: Comm::solo_all_reduce
     p.valid = true;
     return p;
   }

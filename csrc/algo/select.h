@@ -62,6 +62,9 @@ struct Plan {
   const char* reason = "";  // why the plan is invalid
 };
 
+// Whether a collective exists for these types: equal ones with any operator, the mixed triples with Sum / Avg.
+bool triple_ok(DType in, DType wire, DType out, RedOp op);
+
 // Throws nothing; returns plan.valid == false when no kernel can serve the
 // request (caller falls back or reports InvalidArgument).
 Plan make_plan(const PlanInput& in, const CommCaps& caps, const Config& cfg);

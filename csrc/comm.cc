@@ -90,6 +90,13 @@ unsigned long long allocation_id(const void* p) {
 
 MemKind classify(const void* p, bool has_gpu) {
   if (!has_gpu) return MemKind::PlainHost;
+  // One attribute instead of the whole cudaPointerAttributes record: this runs twice per call.
+  const CudaDriver* d = CudaDriver::get();
+  CUmemorytype type = static_cast<CUmemorytype>(0);
+  if (d && d->PointerGetAttribute &&
+      d->PointerGetAttribute(&type, CU_POINTER_ATTRIBUTE_MEMORY_TYPE, reinterpret_cast<CUdeviceptr>(p)) == CUDA_SUCCESS &&
+      type == CU_MEMORYTYPE_DEVICE)
+    return MemKind::Device;
   cudaPointerAttributes a;
   if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
     (void)cudaGetLastError();
@@ -565,6 +572,11 @@ Comm::~Comm() {
       cudaEventDestroy(pipe_->ev_comm[h]);
       cudaEventDestroy(pipe_->ev_out[h]);
     }
+    for (int h = 0; h < kSoloSlots; ++h) {
+      if (pipe_->ev_filled[h]) cudaEventDestroy(pipe_->ev_filled[h]);
+      if (pipe_->ev_work[h]) cudaEventDestroy(pipe_->ev_work[h]);
+      if (pipe_->ev_done[h]) cudaEventDestroy(pipe_->ev_done[h]);
+    }
     pipe_.reset();
   }
   if (solo_stage_) {
@@ -647,7 +659,7 @@ void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType r
   pi.forced = forced;
   size_t in_off = 0, out_off = 0;
   std::shared_ptr<Segment> in_seg, out_seg;
-  if (size_ > 1) {
+  {
     in_seg = find_segment(send, in_bytes, &in_off);
     out_seg = find_segment(recv, out_bytes, &out_off);
     // A registered buffer that was freed and whose address range now belongs to another allocation: the
@@ -705,19 +717,12 @@ void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType r
   const bool host_out = recv_kind == MemKind::PinnedHost;
   bool host_pipe = mode == Mode::AllReduce && (host_in || host_out) && cfg_.host_pipeline_min_bytes != 0 &&
                    std::max(in_bytes, out_bytes) >= cfg_.host_pipeline_min_bytes;
-  if (host_pipe && (!pipe_ || (size_ == 1 && solo_stage_ == nullptr))) {
-    // The first pipelined call creates streams, events and (one rank) device staging: not while a
-    // graph is being captured.  Such a call takes the direct kernel instead.
+  if (host_pipe && !pipe_) {
+    // The first pipelined call creates streams and events: not while a graph is being captured.  Such a
+    // call takes the direct kernel instead.
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) (void)cudaGetLastError();
     if (cs == cudaStreamCaptureStatusActive) host_pipe = false;
-  }
-  if (host_pipe && size_ == 1) {
-    launch_solo_host(send, send_t, recv, recv_t, count, scale, stream, host_in, host_out);  // one rank: Avg == Sum
-    stats_.calls++;
-    stats_.bytes += in_bytes;
-    stats_.pipelined++;
-    return;
   }
   // Ordinary device buffers of the peer-to-peer two-shot AllReduce: export what is new, map what the
   // peers have exported, and let the kernel go direct as soon as every rank can (twoshot_auto_body).
@@ -794,11 +799,7 @@ void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType r
     if (plan.copy_in || plan.copy_out) stats_.staged_passes++;
   }
   if (plan.spec.algo == Algo::Pipe) stats_.staged_passes++;
-  if (size_ == 1 && mode == Mode::AllReduce && send == recv && send_t == recv_t && factor == 1.0) {
-    // Nothing to do; keep stream order semantics without a launch.
-  } else {
-    RT_CHECK(launch_collective(plan.spec, kp, stream), "kernel launch");
-  }
+  RT_CHECK(launch_collective(plan.spec, kp, stream), "kernel launch");
   stats_.calls++;
   stats_.bytes += in_bytes;
   stats_.by_algo[static_cast<int>(plan.spec.algo)]++;
@@ -824,6 +825,11 @@ void Comm::ensure_pipeline() {
       RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_in[h], cudaEventDisableTiming), "cudaEventCreate");
       RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_comm[h], cudaEventDisableTiming), "cudaEventCreate");
       RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_out[h], cudaEventDisableTiming), "cudaEventCreate");
+    }
+    for (int h = 0; size_ == 1 && h < kSoloSlots; ++h) {
+      RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_filled[h], cudaEventDisableTiming), "cudaEventCreate");
+      RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_work[h], cudaEventDisableTiming), "cudaEventCreate");
+      RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_done[h], cudaEventDisableTiming), "cudaEventCreate");
     }
   }
 }
@@ -851,25 +857,15 @@ void Comm::launch_pipelined(const void* send, DType send_t, void* recv, DType re
   const double factor = scale * (op == RedOp::Avg ? 1.0 / static_cast<double>(size_) : 1.0);
 
   auto local_copy = [&](const void* src, DType st, void* dst, DType dt, size_t n, cudaStream_t s) {
-    LaunchSpec ls;
-    ls.algo = Algo::Local;
-    ls.in = st;
-    ls.wire = (st == dt) ? st : DType::Bfloat16;  // the mixed triples all travel as bf16
-    ls.out = dt;
-    ls.op = RedOp::Sum;
-    ls.nthreads = 512;
-    const size_t vecs = (n * std::max(dtype_size(st), dtype_size(dt)) + 15) / 16;
-    ls.nblocks = static_cast<int>(std::min<size_t>(std::max<size_t>(vecs / 2048, 1), 48));
-    KParams kp;
-    memset(&kp, 0, sizeof(kp));
-    kp.comm = dev_;
-    kp.args.send = src;
-    kp.args.recv = dst;
-    kp.args.count = n;
-    kp.args.scale_f = 1.0f;
-    kp.args.scale_d = 1.0;
-    if (!kernel_exists(ls)) fail(Result::InvalidArgument, "no copy kernel for this type combination");
-    RT_CHECK(launch_collective(ls, kp, s), "copy kernel launch");
+    LocalArgs la{};
+    la.send = src;
+    la.recv = dst;
+    la.count = n;
+    la.scale_f = 1.0f;
+    la.scale_d = 1.0;
+    la.identity = 1;
+    if (!local_kernel_exists(st, dt)) fail(Result::InvalidArgument, "no copy kernel for this type combination");
+    RT_CHECK(launch_local(st, dt, la, 96, s), "copy kernel launch");  // half of the SMs' block slots stay free for the collective
   };
 
   RT_CHECK(cudaEventRecord(pipe_->ev_start, stream), "cudaEventRecord");
@@ -946,78 +942,136 @@ void Comm::launch_pipelined(const void* send, DType send_t, void* recv, DType re
   if (i >= 2) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_out[1], 0), "cudaStreamWaitEvent");
 }
 
-// One rank, pinned host buffers: out = factor * in with the types converted, as a three-stage
-// pipeline through private device staging: copy engine in, kernel, copy engine out.  Host -> device
-// and device -> host run at the same time (PCIe is full duplex).
-void Comm::launch_solo_host(const void* send, DType send_t, void* recv, DType recv_t, size_t count, double factor,
-                            cudaStream_t stream, bool host_in, bool host_out) {
+// One rank: out = scale * in with the types converted; every operator is the identity.  Device buffers
+// take one kernel (k_local.cu).  Pinned host buffers, by size:
+//   below two pipeline chunks (16 MB)  the same kernel reads and writes host memory itself, capped at 32
+//                                      blocks: PCIe carries both directions at once from the first byte
+//                                      (4 MiB of fp32: 112 us with 32 blocks, 151 us with 148, 167 us as
+//                                      copy in, kernel, copy out)
+//   from there on                      a chunk pipeline of copy engine in (, kernel), copy engine out
+//                                      (32 MiB: 842 us either way; 256 MiB: 6.1 against 6.7 ms)
+void Comm::solo_all_reduce(const void* send, DType send_t, void* recv, DType recv_t, DType wire_t, size_t count, RedOp op,
+                           double scale, cudaStream_t stream) {
+  const bool is_float = send_t == DType::Float16 || send_t == DType::Bfloat16 || send_t == DType::Float32 || send_t == DType::Float64;
+  if (!is_float && scale != 1.0) fail(Result::InvalidArgument, "a scale factor needs a floating-point type");
+  const size_t in_bytes = count * dtype_size(send_t), out_bytes = count * dtype_size(recv_t);
+  const MemKind send_kind = classify(send, true);
+  const MemKind recv_kind = recv == send ? send_kind : classify(recv, true);
+  if (send_kind == MemKind::PlainHost || recv_kind == MemKind::PlainHost)
+    fail(Result::InvalidArgument, "buffers must be device memory or pinned host memory on the GPU data plane");
+  if (!triple_ok(send_t, wire_t, recv_t, op))
+    fail(Result::InvalidArgument, "no kernel for this request: unsupported (send, wire, recv) type combination for this operator");
+  NvtxDomainRange nvtx_range("allreduce/local", in_bytes);
+  const bool host_in = send_kind == MemKind::PinnedHost, host_out = recv_kind == MemKind::PinnedHost;
+  LocalArgs la{};
+  la.send = send;
+  la.recv = recv;
+  la.count = count;
+  la.scale_f = static_cast<float>(scale);
+  la.scale_d = scale;
+  la.identity = scale == 1.0 ? 1 : 0;
+  stats_.calls++;
+  stats_.bytes += in_bytes;
+  const bool in_place = send == recv && send_t == recv_t && la.identity;  // nothing to do
+  if ((host_in || host_out) && !in_place) {
+    // The first pipelined call creates streams, events and device staging: not while a graph is being
+    // captured.  Such a call takes the kernel instead.
+    const size_t bytes = std::max(in_bytes, out_bytes);
+    bool pipeline = cfg_.host_pipeline_min_bytes != 0 && bytes >= std::max(cfg_.host_pipeline_min_bytes, 2 * cfg_.host_chunk_bytes);
+    if (pipeline && (!pipe_ || solo_slot_bytes_ < solo_chunk_bytes(SIZE_MAX))) {
+      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+      if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) (void)cudaGetLastError();
+      if (cs == cudaStreamCaptureStatusActive) pipeline = false;
+    }
+    if (pipeline) {
+      launch_solo_host(la, send_t, recv_t, stream, host_in, host_out);
+      stats_.pipelined++;
+      return;
+    }
+  }
+  if (!in_place) RT_CHECK(launch_local(send_t, recv_t, la, host_in || host_out ? 32 : 0, stream), "kernel launch");
+  stats_.by_algo[static_cast<int>(Algo::Local)]++;
+}
+
+// Chunk of the one-rank host pipeline: an eighth of the message, between half and twice the configured
+// chunk.  Small chunks shorten the first copy in and the last copy out, which nothing overlaps, but every
+// hand-over from engine to engine costs about 10 us (B200, ms: 64 MiB 1.63 / 1.61 / 1.69 with 4 / 8 / 16 MB,
+// 256 MiB 6.48 / 6.24 / 6.14).
+size_t Comm::solo_chunk_bytes(size_t bytes) const {
+  const size_t c = std::min(std::max(bytes / 8, cfg_.host_chunk_bytes / 2), 2 * cfg_.host_chunk_bytes);
+  return std::max<size_t>((c + 65535) & ~size_t(65535), 65536);
+}
+
+// One rank, pinned host buffers, as a pipeline through a ring of device slots: copy engine in, kernel (only
+// where something is scaled or converted), copy engine out.  Host -> device and device -> host run at the
+// same time (PCIe is full duplex).
+void Comm::launch_solo_host(const LocalArgs& call, DType send_t, DType recv_t, cudaStream_t stream, bool host_in, bool host_out) {
   ensure_pipeline();
-  const size_t isz = dtype_size(send_t), osz = dtype_size(recv_t);
-  size_t chunk = cfg_.host_chunk_bytes / std::max(isz, osz);
-  chunk &= ~size_t(4095);
-  if (chunk == 0) chunk = 4096;
-  const size_t half = (std::max(cfg_.host_chunk_bytes, chunk * std::max(isz, osz)) + 255) & ~size_t(255);  // the same for every type
-  if (solo_stage_ == nullptr || solo_stage_half_ < half) {
+  const size_t isz = dtype_size(send_t), osz = dtype_size(recv_t), wide = std::max(isz, osz);
+  // Slots for the largest chunk from the start: a captured call keeps their addresses.
+  const size_t slot = solo_chunk_bytes(SIZE_MAX);
+  if (solo_stage_ == nullptr || solo_slot_bytes_ < slot) {
     if (solo_stage_) {
       RT_CHECK(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
       cudaFree(solo_stage_);
       solo_stage_ = nullptr;
+      solo_slot_bytes_ = 0;
     }
-    RT_CHECK(cudaMalloc(reinterpret_cast<void**>(&solo_stage_), 4 * half), "cudaMalloc (host staging)");
-    solo_stage_half_ = half;
+    RT_CHECK(cudaMalloc(reinterpret_cast<void**>(&solo_stage_), kSoloSlots * slot), "cudaMalloc (host staging)");
+    solo_slot_bytes_ = slot;
   }
-  LaunchSpec ls;
-  ls.algo = Algo::Local;
-  ls.in = send_t;
-  ls.wire = (send_t == recv_t) ? send_t : DType::Bfloat16;
-  ls.out = recv_t;
-  ls.op = RedOp::Sum;
-  ls.nthreads = 512;
-  if (!kernel_exists(ls)) fail(Result::InvalidArgument, "no kernel for this type combination");
+  const size_t chunk = solo_chunk_bytes(call.count * wide) / wide;
+  const bool kernel = !(send_t == recv_t && call.identity);
+  // slots: all of them hold input on its way to the output, or half of them inputs and half results
+  const int ring = kernel ? kSoloSlots / 2 : kSoloSlots;
+  char* const out_slots = solo_stage_ + (kernel ? ring * solo_slot_bytes_ : 0);
   // only the side streams that get work are forked (a forked stream must be joined under capture)
   RT_CHECK(cudaEventRecord(pipe_->ev_start, stream), "cudaEventRecord");
   if (host_in) RT_CHECK(cudaStreamWaitEvent(pipe_->s_in, pipe_->ev_start, 0), "cudaStreamWaitEvent");
   if (host_out) RT_CHECK(cudaStreamWaitEvent(pipe_->s_out, pipe_->ev_start, 0), "cudaStreamWaitEvent");
-  size_t i = 0;
-  for (size_t off = 0; off < count; off += chunk, ++i) {
-    const int h = static_cast<int>(i & 1);
-    const size_t n = std::min(chunk, count - off);
-    char* a_h = solo_stage_ + h * half;
-    char* b_h = solo_stage_ + (2 + h) * half;
-    const char* src = static_cast<const char*>(send) + off * isz;
-    char* dst = static_cast<char*>(recv) + off * osz;
-    const void* k_in = src;
+  int i = 0;
+  for (size_t off = 0; off < call.count; off += chunk, ++i) {
+    const int h = i % ring;
+    const size_t n = std::min(chunk, call.count - off);
+    const char* src = static_cast<const char*>(call.send) + off * isz;
+    char* dst = static_cast<char*>(call.recv) + off * osz;
+    const char* k_in = src;      // what the kernel (or the copy out) reads
+    cudaStream_t last = stream;  // where the result of this chunk is produced
     if (host_in) {
-      if (i >= 2) RT_CHECK(cudaStreamWaitEvent(pipe_->s_in, pipe_->ev_comm[h], 0), "cudaStreamWaitEvent");
+      char* a_h = (!kernel && !host_out) ? dst : solo_stage_ + h * solo_slot_bytes_;   // host -> device, nothing to convert: straight in
+      // the slot's last reader: the kernel, or the copy out of a pipeline without one
+      if (i >= ring && (kernel || host_out))
+        RT_CHECK(cudaStreamWaitEvent(pipe_->s_in, kernel ? pipe_->ev_work[h] : pipe_->ev_done[h], 0), "cudaStreamWaitEvent");
       RT_CHECK(cudaMemcpyAsync(a_h, src, n * isz, cudaMemcpyHostToDevice, pipe_->s_in), "cudaMemcpyAsync");
-      RT_CHECK(cudaEventRecord(pipe_->ev_in[h], pipe_->s_in), "cudaEventRecord");
-      RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_in[h], 0), "cudaStreamWaitEvent");
+      RT_CHECK(cudaEventRecord(pipe_->ev_filled[h], pipe_->s_in), "cudaEventRecord");
       k_in = a_h;
+      last = pipe_->s_in;
     }
-    if (host_out && i >= 2) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_out[h], 0), "cudaStreamWaitEvent");
-    KParams kp;
-    memset(&kp, 0, sizeof(kp));
-    kp.comm = dev_;
-    kp.args.send = k_in;
-    kp.args.recv = host_out ? static_cast<void*>(b_h) : static_cast<void*>(dst);
-    kp.args.count = n;
-    kp.args.scale_f = static_cast<float>(factor);
-    kp.args.scale_d = factor;
-    const size_t vecs = (n * std::max(isz, osz) + 15) / 16;
-    ls.nblocks = static_cast<int>(std::min<size_t>(std::max<size_t>(vecs / 2048, 1), 96));
-    RT_CHECK(launch_collective(ls, kp, stream), "kernel launch");
-    RT_CHECK(cudaEventRecord(pipe_->ev_comm[h], stream), "cudaEventRecord");
+    if (kernel) {
+      char* b_h = host_out ? out_slots + h * solo_slot_bytes_ : dst;
+      if (host_in) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_filled[h], 0), "cudaStreamWaitEvent");
+      if (host_out && i >= ring) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_done[h], 0), "cudaStreamWaitEvent");
+      LocalArgs la = call;
+      la.send = k_in;
+      la.recv = b_h;
+      la.count = n;
+      RT_CHECK(launch_local(send_t, recv_t, la, 0, stream), "kernel launch");
+      RT_CHECK(cudaEventRecord(pipe_->ev_work[h], stream), "cudaEventRecord");
+      k_in = b_h;
+      last = stream;
+    }
     if (host_out) {
-      RT_CHECK(cudaStreamWaitEvent(pipe_->s_out, pipe_->ev_comm[h], 0), "cudaStreamWaitEvent");
-      RT_CHECK(cudaMemcpyAsync(dst, b_h, n * osz, cudaMemcpyDeviceToHost, pipe_->s_out), "cudaMemcpyAsync");
-      RT_CHECK(cudaEventRecord(pipe_->ev_out[h], pipe_->s_out), "cudaEventRecord");
+      if (last != stream || kernel)
+        RT_CHECK(cudaStreamWaitEvent(pipe_->s_out, kernel ? pipe_->ev_work[h] : pipe_->ev_filled[h], 0), "cudaStreamWaitEvent");
+      RT_CHECK(cudaMemcpyAsync(dst, k_in, n * osz, cudaMemcpyDeviceToHost, pipe_->s_out), "cudaMemcpyAsync");
+      RT_CHECK(cudaEventRecord(pipe_->ev_done[h], pipe_->s_out), "cudaEventRecord");
     }
   }
   stats_.by_algo[static_cast<int>(Algo::Local)]++;
-  if (host_out) {
-    RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_out[0], 0), "cudaStreamWaitEvent");
-    if (i >= 2) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_out[1], 0), "cudaStreamWaitEvent");
-  }
+  // the side streams run in order: their last event stands for all of their work
+  const int h = (i - 1) % ring;
+  if (host_out) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_done[h], 0), "cudaStreamWaitEvent");
+  else RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_filled[h], 0), "cudaStreamWaitEvent");
 }
 
 void Comm::wait_blocking(cudaStream_t stream) {
@@ -1074,7 +1128,8 @@ void Comm::all_reduce(const void* send, DType send_t, void* recv, DType recv_t, 
   }
   if (forced == Algo::Auto) forced = parse_algo(cfg_.algo);
   if (forced == Algo::Ring) forced = Algo::Auto;
-  launch(Mode::AllReduce, send, send_t, recv, recv_t, wire_t, count, op, scale, forced, stream);
+  if (size_ == 1) solo_all_reduce(send, send_t, recv, recv_t, wire_t, count, op, scale, stream);
+  else launch(Mode::AllReduce, send, send_t, recv, recv_t, wire_t, count, op, scale, forced, stream);
   if (cfg_.blocking && !capturing) wait_blocking(stream);
 }
 
@@ -1083,7 +1138,7 @@ void Comm::reduce_scatter(const void* send, void* recv, size_t recvcount, DType 
   check_usable();
   if (!gpu_plane_) fail(Result::InvalidUsage, "ReduceScatter needs the GPU data plane");
   if (size_ == 1) {
-    launch(Mode::AllReduce, send, t, recv, t, t, recvcount, op, 1.0, Algo::Auto, stream);
+    solo_all_reduce(send, t, recv, t, t, recvcount, op, 1.0, stream);
     return;
   }
   launch(Mode::ReduceScatter, send, t, recv, t, t, recvcount, op, 1.0, parse_algo(cfg_.algo), stream);

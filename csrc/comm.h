@@ -89,8 +89,10 @@ class Comm {
               RedOp op, double scale, Algo forced, cudaStream_t stream);
   void launch_pipelined(const void* send, DType send_t, void* recv, DType recv_t, DType wire_t, size_t count, RedOp op,
                         double scale, Algo forced, cudaStream_t stream, bool host_in = false, bool host_out = false);
-  void launch_solo_host(const void* send, DType send_t, void* recv, DType recv_t, size_t count, double factor,
-                        cudaStream_t stream, bool host_in, bool host_out);
+  void solo_all_reduce(const void* send, DType send_t, void* recv, DType recv_t, DType wire_t, size_t count, RedOp op,
+                       double scale, cudaStream_t stream);
+  void launch_solo_host(const LocalArgs& call, DType send_t, DType recv_t, cudaStream_t stream, bool host_in, bool host_out);
+  size_t solo_chunk_bytes(size_t bytes) const;
   void ensure_pipeline();
   void ring_all_reduce(const void* send, void* recv, size_t count, DType t, RedOp op, cudaStream_t stream);
   void init_shared_gpu_plane();
@@ -149,14 +151,16 @@ class Comm {
   void auto_import();                        // map what the peers have exported since the last look
 
   // chunk pipeline for large AllReduces on ordinary buffers
+  static constexpr int kSoloSlots = 8;
   struct Pipeline {
     cudaStream_t s_in = nullptr, s_out = nullptr;
     cudaEvent_t ev_start = nullptr, ev_in[2] = {nullptr, nullptr}, ev_comm[2] = {nullptr, nullptr}, ev_out[2] = {nullptr, nullptr};
+    cudaEvent_t ev_filled[kSoloSlots] = {}, ev_work[kSoloSlots] = {}, ev_done[kSoloSlots] = {};  // one rank only
   };
   std::unique_ptr<Pipeline> pipe_;
-  // single rank with pinned-host buffers: private device staging (two halves per direction)
+  // single rank with pinned-host buffers: private device staging, a ring of kSoloSlots chunks
   char* solo_stage_ = nullptr;
-  size_t solo_stage_half_ = 0;
+  size_t solo_slot_bytes_ = 0;
 
   // plane for ranks that share a GPU: host-synchronised, staging exchanged over CUDA IPC
   bool shared_plane_ = false;

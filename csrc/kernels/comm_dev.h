@@ -129,6 +129,16 @@ struct CollArgs {
   AutoDesc auto_desc;        // twoshot_auto_body: what this rank tells its peers about the call
 };
 
+// Arguments of the one-rank kernel (k_local.cu): out[i] = scale * in[i], types converted.
+struct LocalArgs {
+  const void* send;
+  void* recv;
+  uint64_t count;
+  float scale_f;             // factor for fp16 / bf16 / fp32
+  int32_t identity;          // factor 1 (always so for integer types): equal types are copied as they are
+  double scale_d;            // the factor for fp64
+};
+
 struct KParams {
   CommDev comm;
   CollArgs args;

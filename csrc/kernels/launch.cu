@@ -4,7 +4,6 @@
 
 namespace mnccl {
 namespace dev {
-cudaError_t dispatch_local(const LaunchCtx&);
 cudaError_t dispatch_ll(const LaunchCtx&);
 cudaError_t dispatch_oneshot(const LaunchCtx&);
 cudaError_t dispatch_twoshot_ar(const LaunchCtx&);
@@ -24,7 +23,6 @@ cudaError_t route(const dev::LaunchCtx& x) {
   switch (s.mode) {
     case Mode::AllReduce:
       switch (s.algo) {
-        case Algo::Local: return dev::dispatch_local(x);
         case Algo::LL: return dev::dispatch_ll(x);
         case Algo::OneShot: return dev::dispatch_oneshot(x);
         case Algo::TwoShot: return s.auto_direct ? dev::dispatch_twoshot_auto(x) : dev::dispatch_twoshot_ar(x);
@@ -52,7 +50,7 @@ bool kernel_exists(const LaunchSpec& spec) {
 
 cudaError_t launch_collective(const LaunchSpec& spec, const KParams& p, cudaStream_t stream) {
   // Only kernels with per-block barrier state are bound by kMaxBlocks.
-  const int max_blocks = (spec.algo == Algo::Local || spec.algo == Algo::HostSync) ? 65535 : kMaxBlocks;
+  const int max_blocks = spec.algo == Algo::HostSync ? 65535 : kMaxBlocks;
   if (spec.nblocks < 1 || spec.nblocks > max_blocks || spec.nthreads < 32 || spec.nthreads > 512)
     return cudaErrorInvalidConfiguration;
   if (spec.auto_direct && spec.nblocks > kAutoBlocks) return cudaErrorInvalidConfiguration;

@@ -38,6 +38,10 @@ bool kernel_exists(const LaunchSpec& spec);
 // Launch on one rank (the normal case).  `p` is passed by value to the kernel.
 cudaError_t launch_collective(const LaunchSpec& spec, const KParams& p, cudaStream_t stream);
 
+// One rank (k_local.cu): a copy with scale and cast.  `max_blocks` caps the grid (0 = one block per tile).
+bool local_kernel_exists(DType in, DType out);
+cudaError_t launch_local(DType in, DType out, const LocalArgs& a, int max_blocks, cudaStream_t stream);
+
 // Single-GPU emulation of `vranks` ranks: ONE cooperative launch whose grid is
 // vranks * spec.nblocks blocks; block g acts as block g % nblocks of rank
 // g / nblocks and reads its parameters from table[g / nblocks] (device
