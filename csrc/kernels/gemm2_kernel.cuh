@@ -113,6 +113,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   const uint32_t tmem_base = ctl->tmem_base;
   const uint32_t epoch = ctl->epoch;
   const uint64_t budget = g.wait_budget_ns;
+  const bool leader = elect_one();  // the lane that issues for its warp (producer and MMA roles)
 
   // 256-row tile index -> (tm2, tn); this CTA's 128 rows are tile 2 * tm2 + cta of the
   // 128-row numbering the epilogues use.
@@ -122,75 +123,55 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int t = pair; t < num_items && ok; t += n_pairs) {
-        const PairWork w = pair_work(g, t, num_kb);
-        int tm2, tn;
-        tile_coords(g2, w.tile, tiles_m2, tiles_n, &tm2, &tn);
-        const int tm = tm2 * 2 + static_cast<int>(cta);
-        if (g.a_ready != nullptr) {
-          const int chunk = (tm * kBM) / g.rows_per_chunk;
-          const int last_chunk = (min(tm * kBM + kBM, g.M) - 1) / g.rows_per_chunk;
-          const uint32_t target = epoch * g.a_ready_mult;
-          bool waited = false;
-          for (int c = chunk; c <= last_chunk && ok; ++c) {
-            if (c >= g.a_local_first && c < g.a_local_first + g.a_local_count) continue;
-            waited = true;
-            const uint64_t t0 = globaltimer_ns();
-            uint32_t spins = 0;
-            while (static_cast<int32_t>(ld_acquire_sys_u32(g.a_ready + c) - target) < 0) {
-              if ((++spins & 255u) == 0u && (comm_aborted(g) || ctl->abort != 0u || globaltimer_ns() - t0 > budget)) {
-                if (ctl->abort == 0u) ctl->abort = comm_aborted(g) ? kGemmAborted : kGemmRowsTimeout;
-                ok = false;
-                break;
-              }
-            }
-          }
-          if (!ok) break;
-          if (waited) asm volatile("fence.proxy.async.global;" ::: "memory");
-        }
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
-          const uint32_t s = it % NS;
-          const uint32_t ph = (it / NS) & 1u;
-          if (!mbar_wait(smem_u32(&ctl->empty[s]), ph ^ 1u, &ctl->abort, budget)) { ok = false; break; }
-          const uint32_t leader_full = map_to_cta(smem_u32(&ctl->full[s]), 0);
-          mbar_arrive_expect_tx_cluster(leader_full, k2StageBytes);
+    uint32_t s = 0, ph = 1;
+    bool ok = true;
+    const uint32_t leader_full = map_to_cta(smem_u32(&ctl->full[0]), 0);
+    for (int t = pair; t < num_items && ok; t += n_pairs) {
+      const PairWork w = pair_work(g, t, num_kb);
+      int tm2, tn;
+      tile_coords(g2, w.tile, tiles_m2, tiles_n, &tm2, &tn);
+      const int tm = tm2 * 2 + static_cast<int>(cta);
+      if (g.a_ready != nullptr && !rows_ready(g, epoch, tm, leader, &ctl->abort)) { ok = false; break; }
+      for (int kb = w.kb0; kb < w.kb1; ++kb) {
+        if (!mbar_wait_warp(smem_u32(&ctl->empty[0]) + s * 8u, ph, &ctl->abort, budget)) { ok = false; break; }
+        if (leader) {
+          const uint32_t full = leader_full + s * 8u;
+          mbar_arrive_expect_tx_cluster(full, k2StageBytes);
           const uint32_t sa = base + s * k2StageBytes;
-          tma_load_2d_pair(sa, &tma_a, leader_full, kb * kBK, tm * kBM);
-          tma_load_2d_pair(sa + kTileABytes, &tma_b, leader_full, kb * kBK, tn * kBN + static_cast<int>(cta) * (kBN / 2));
+          tma_load_2d_pair(sa, &tma_a, full, kb * kBK, tm * kBM);
+          tma_load_2d_pair(sa + kTileABytes, &tma_b, full, kb * kBK, tn * kBN + static_cast<int>(cta) * (kBN / 2));
         }
+        if (++s == NS) { s = 0; ph ^= 1u; }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && cta == 0) {
+    if (cta == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(2 * kBM, kBN);
-      uint32_t it = 0, local = 0;
+      const uint64_t da0 = make_smem_desc_sw128(base), db0 = make_smem_desc_sw128(base + kTileABytes);
+      uint32_t s = 0, ph = 0, local = 0;
       bool ok = true;
       for (int t = pair; t < num_items && ok; t += n_pairs, ++local) {
         const PairWork w = pair_work(g, t, num_kb);
         const uint32_t buf = local & 1u;
         const uint32_t acc_ph = (local >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&ctl->tmem_empty[buf]), acc_ph ^ 1u, &ctl->abort, budget)) { ok = false; break; }
+        if (!mbar_wait_warp(smem_u32(&ctl->tmem_empty[0]) + buf * 8u, acc_ph ^ 1u, &ctl->abort, budget)) { ok = false; break; }
         tc_fence_after_sync();
         const uint32_t d = tmem_base + buf * kBN;
-        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
-          const uint32_t s = it % NS;
-          const uint32_t ph = (it / NS) & 1u;
-          if (!mbar_wait(smem_u32(&ctl->full[s]), ph, &ctl->abort, budget)) { ok = false; break; }
+        for (int kb = w.kb0; kb < w.kb1; ++kb) {
+          if (!mbar_wait_warp(smem_u32(&ctl->full[0]) + s * 8u, ph, &ctl->abort, budget)) { ok = false; break; }
           tc_fence_after_sync();
-          const uint32_t sa = base + s * k2StageBytes;
-          const uint64_t da = make_smem_desc_sw128(sa);
-          const uint64_t db = make_smem_desc_sw128(sa + kTileABytes);
+          const uint64_t da = da0 + static_cast<uint64_t>(s * (k2StageBytes >> 4)), db = db0 + static_cast<uint64_t>(s * (k2StageBytes >> 4));
+          if (leader) {
 #pragma unroll
-          for (int k = 0; k < kBK / kUmmaK; ++k)
-            umma_bf16_pair(d, da + static_cast<uint64_t>(k * 2), db + static_cast<uint64_t>(k * 2), idesc,
-                           ((kb - w.kb0) | k) != 0 ? 1u : 0u);
-          umma_commit_pair(smem_u32(&ctl->empty[s]), 3);  // the stage is free in both CTAs
+            for (int k = 0; k < kBK / kUmmaK; ++k)
+              umma_bf16_pair(d, da + static_cast<uint64_t>(k * 2), db + static_cast<uint64_t>(k * 2), idesc,
+                             ((kb - w.kb0) | k) != 0 ? 1u : 0u);
+            umma_commit_pair(smem_u32(&ctl->empty[0]) + s * 8u, 3);  // the stage is free in both CTAs
+          }
+          if (++s == NS) { s = 0; ph ^= 1u; }
         }
-        if (ok) umma_commit_pair(smem_u32(&ctl->tmem_full[buf]), 3);
+        if (ok && leader) umma_commit_pair(smem_u32(&ctl->tmem_full[0]) + buf * 8u, 3);
       }
     }
   } else {

@@ -68,6 +68,37 @@ __device__ __forceinline__ bool finish_epoch(const GemmArgs& g, uint32_t epoch) 
 // True when the communicator's abort word is set (polled by every wait on a peer).
 __device__ __forceinline__ bool comm_aborted(const GemmArgs& g) { return g.comm_abort != nullptr && *g.comm_abort != 0u; }
 
+// all-gather -> GEMM: waits (bounded) until the rows of 128-row tile `tm` have arrived.  One lane polls, the
+// whole warp gets the answer.
+__device__ __forceinline__ bool rows_ready(const GemmArgs& g, uint32_t epoch, int tm, bool leader, volatile uint32_t* abort_flag) {
+  bool ok = true;
+  if (leader) {
+    const int first = (tm * kBM) / g.rows_per_chunk;
+    const int last = (min(tm * kBM + kBM, g.M) - 1) / g.rows_per_chunk;
+    const uint32_t target = epoch * g.a_ready_mult;
+    bool waited = false;
+    for (int c = first; c <= last && ok; ++c) {
+      if (c >= g.a_local_first && c < g.a_local_first + g.a_local_count) continue;  // rows that never left this GPU
+      waited = true;
+      const uint64_t t0 = globaltimer_ns();
+      uint32_t spins = 0;
+      while (static_cast<int32_t>(ld_acquire_sys_u32(g.a_ready + c) - target) < 0) {
+        if ((++spins & 255u) == 0u) {
+          const bool aborted = comm_aborted(g);
+          if (aborted || *abort_flag != 0u || globaltimer_ns() - t0 > g.wait_budget_ns) {
+            if (*abort_flag == 0u) *abort_flag = aborted ? kGemmAborted : kGemmRowsTimeout;
+            ok = false;
+            break;
+          }
+        }
+      }
+    }
+    // rows written by a peer's generic stores are about to be read by the async proxy
+    if (ok && waited) asm volatile("fence.proxy.async.global;" ::: "memory");
+  }
+  return __all_sync(0xffffffffu, ok) != 0;
+}
+
 struct __align__(8) SharedCtl {
   uint64_t full[kStages];
   uint64_t empty[kStages];
@@ -150,93 +181,66 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   const uint32_t tmem_base = ctl->tmem_base;
   const uint32_t epoch = ctl->epoch;
   const uint64_t budget = g.wait_budget_ns;
+  const bool leader = elect_one();  // the lane that issues for its warp (producer and MMA roles)
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      uint32_t it = 0;  // ring position over all k-blocks of all my tiles
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += n_gemm) {
-        int tm, tn;
-        tile_coords(g, t, tiles_m, tiles_n, &tm, &tn);
-        // all-gather -> GEMM: the rows of this tile may still be on their way
-        if (g.a_ready != nullptr) {
-          const int chunk = (tm * kBM) / g.rows_per_chunk;
-          const int last_chunk = (min(tm * kBM + kBM, g.M) - 1) / g.rows_per_chunk;
-          const uint32_t target = epoch * g.a_ready_mult;
-          bool waited = false;
-          for (int c = chunk; c <= last_chunk && ok; ++c) {
-            if (c >= g.a_local_first && c < g.a_local_first + g.a_local_count) continue;  // rows that never left this GPU
-            waited = true;
-            const uint64_t t0 = globaltimer_ns();
-            uint32_t spins = 0;
-            while (static_cast<int32_t>(ld_acquire_sys_u32(g.a_ready + c) - target) < 0) {
-              if ((++spins & 255u) == 0u) {
-                const bool aborted = comm_aborted(g);
-                if (aborted || ctl->abort != 0u || globaltimer_ns() - t0 > budget) {
-                  if (ctl->abort == 0u) ctl->abort = aborted ? kGemmAborted : kGemmRowsTimeout;
-                  ok = false;
-                  break;
-                }
-              }
-            }
-          }
-          if (!ok) break;
-          // rows written by a peer's generic stores are about to be read by the async proxy
-          if (waited) asm volatile("fence.proxy.async.global;" ::: "memory");
-        }
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const uint32_t s = it % NS;
-          const uint32_t ph = (it / NS) & 1u;
-          if (!mbar_wait(smem_u32(&ctl->empty[s]), ph ^ 1u, &ctl->abort, budget)) { ok = false; break; }
-          const uint32_t full = smem_u32(&ctl->full[s]);
+    uint32_t it = 0, s = 0, ph = 1;  // ring position over all k-blocks of all my tiles: count, stage, parity to wait for
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += n_gemm) {
+      int tm, tn;
+      tile_coords(g, t, tiles_m, tiles_n, &tm, &tn);
+      // all-gather -> GEMM: the rows of this tile may still be on their way
+      if (g.a_ready != nullptr && !rows_ready(g, epoch, tm, leader, &ctl->abort)) { ok = false; break; }
+      for (int kb = 0; kb < num_kb; ++kb, ++it) {
+        if (!mbar_wait_warp(smem_u32(&ctl->empty[0]) + s * 8u, ph, &ctl->abort, budget)) { ok = false; break; }
+        if (leader) {
+          const uint32_t full = smem_u32(&ctl->full[0]) + s * 8u;
           mbar_arrive_expect_tx(full, kTileABytes + BN * kBK * 2);
           const uint32_t sa = base + s * kStageBytes;
           tma_load_2d(sa, &tma_a, full, kb * kBK, tm * kBM);
           tma_load_2d(sa + kTileABytes, &tma_b, full, kb * kBK, tn * BN);
         }
+        if (++s == NS) { s = 0; ph ^= 1u; }
       }
-      // Wind-down after a failed wait: let copies that are still in flight land
-      // before the CTA (and its shared memory) goes away.
-      if (!ok) {
-        for (uint32_t back = 0; back < NS && back < it; ++back) {
-          const uint32_t j = it - 1 - back;
-          mbar_wait(smem_u32(&ctl->full[j % NS]), (j / NS) & 1u, &ctl->abort /*already set*/, 0);
-          // (budget 0: one more try each; the data either landed or the MMA side consumed it)
-        }
+    }
+    // Wind-down after a failed wait: let copies that are still in flight land
+    // before the CTA (and its shared memory) goes away.
+    if (!ok) {
+      for (uint32_t back = 0; back < NS && back < it; ++back) {
+        const uint32_t j = it - 1 - back;
+        mbar_wait(smem_u32(&ctl->full[j % NS]), (j / NS) & 1u, &ctl->abort /*already set*/, 0);
+        // (budget 0: one more try each; the data either landed or the MMA side consumed it)
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(kBM, BN);
-      uint32_t it = 0;
-      uint32_t local = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < num_tiles && ok; t += n_gemm, ++local) {
-        const uint32_t buf = local & 1u;
-        const uint32_t acc_ph = (local >> 1) & 1u;
-        if (!mbar_wait(smem_u32(&ctl->tmem_empty[buf]), acc_ph ^ 1u, &ctl->abort, budget)) { ok = false; break; }
+    constexpr uint32_t idesc = make_idesc_bf16(kBM, BN);
+    const uint64_t da0 = make_smem_desc_sw128(base), db0 = make_smem_desc_sw128(base + kTileABytes);
+    uint32_t s = 0, ph = 0, local = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < num_tiles && ok; t += n_gemm, ++local) {
+      const uint32_t buf = local & 1u;
+      const uint32_t acc_ph = (local >> 1) & 1u;
+      if (!mbar_wait_warp(smem_u32(&ctl->tmem_empty[0]) + buf * 8u, acc_ph ^ 1u, &ctl->abort, budget)) { ok = false; break; }
+      tc_fence_after_sync();
+      const uint32_t d = tmem_base + buf * kBN;
+      for (int kb = 0; kb < num_kb; ++kb) {
+        if (!mbar_wait_warp(smem_u32(&ctl->full[0]) + s * 8u, ph, &ctl->abort, budget)) { ok = false; break; }
         tc_fence_after_sync();
-        const uint32_t d = tmem_base + buf * kBN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const uint32_t s = it % NS;
-          const uint32_t ph = (it / NS) & 1u;
-          if (!mbar_wait(smem_u32(&ctl->full[s]), ph, &ctl->abort, budget)) { ok = false; break; }
-          tc_fence_after_sync();
-          const uint32_t sa = base + s * kStageBytes;
-          const uint64_t da = make_smem_desc_sw128(sa);
-          const uint64_t db = make_smem_desc_sw128(sa + kTileABytes);
+        const uint64_t da = da0 + static_cast<uint64_t>(s * (kStageBytes >> 4)), db = db0 + static_cast<uint64_t>(s * (kStageBytes >> 4));
+        if (leader) {
 #pragma unroll
           for (int k = 0; k < kBK / kUmmaK; ++k) {
             // advance 16 elements = 32 bytes inside the 128-byte swizzle row: +2 in the address field
             umma_bf16(d, da + static_cast<uint64_t>(k * 2), db + static_cast<uint64_t>(k * 2), idesc,
                       (kb | k) != 0 ? 1u : 0u);
           }
-          umma_commit(smem_u32(&ctl->empty[s]));  // the stage is free once these MMAs have read it
+          umma_commit(smem_u32(&ctl->empty[0]) + s * 8u);  // the stage is free once these MMAs have read it
         }
-        if (ok) umma_commit(smem_u32(&ctl->tmem_full[buf]));
+        if (++s == NS) { s = 0; ph ^= 1u; }
       }
+      if (ok && leader) umma_commit(smem_u32(&ctl->tmem_full[0]) + buf * 8u);
     }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..5)
