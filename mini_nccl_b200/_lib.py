@@ -96,6 +96,8 @@ def lib() -> C.CDLL:
         sig("mncclGemmStatus", i32, P(u32))
         if hasattr(L, "mncclGemmSetPairMode"):
             sig("mncclGemmSetPairMode", None, i32)
+        if hasattr(L, "mncclGemmSmallPlan"):
+            sig("mncclGemmSmallPlan", i32, i32, i32, i32, i32, i32, P(i32), P(i32), P(i32))
         if hasattr(L, "mncclGemmPlan"):
             sig("mncclGemmPlan", None, i32, i32, i32, i32, C.POINTER(C.c_int), C.POINTER(C.c_int))
     if hasattr(L, "mncclSwiGluBf16"):
@@ -199,7 +201,8 @@ def ext():
     from . import _torch_ext
 
     address = lambda name: C.cast(getattr(L, name), C.c_void_p).value if hasattr(L, name) else 0
-    _torch_ext.bind(address("mncclAllReduceEx"), address("mncclCommGetAsyncError"), address("mncclGemmBf16"))
+    _torch_ext.bind(address("mncclAllReduceEx"), address("mncclCommGetAsyncError"), address("mncclGemmBf16"),
+                    address("mncclGemmReduceScatterBf16Comm"), address("mncclAllGatherGemmBf16Comm"))
     _EXT = _torch_ext
     return _EXT
 

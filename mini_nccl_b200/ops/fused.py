@@ -22,7 +22,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
-from .._lib import lib
+from .._lib import MiniNcclError, ext, lib
 
 BM = 128
 
@@ -49,8 +49,6 @@ def _check_comm(comm):
     """A communicator that has failed (watchdog trip, a kernel's failed wait, abort) takes no more work."""
     err = comm.async_error()
     if err != 0:
-        from .._lib import MiniNcclError
-
         raise MiniNcclError(err, "fused kernel on a failed communicator")
 
 
@@ -88,6 +86,10 @@ class GemmReduceScatter:
             self._mc = comm.peer_pointers(self.stage)[1]
         # CTAs that only sum finished tiles in the switch form (0: the kernel's default of 16)
         self.n_comm_ctas = int(os.environ.get("MINI_NCCL_RS_COMM_CTAS", "0"))
+        self._handle_buf = C.create_string_buffer(self._handle, len(self._handle))
+        self._workspace = (M, N, comm.rank, R, C.addressof(self._stage_peers), C.addressof(self._flag_peers), self.state.data_ptr(),
+                           C.addressof(self._handle_buf), len(self._handle))
+        self._call = ext().gemm_rs
 
     @property
     def in_switch(self) -> bool:
@@ -96,6 +98,14 @@ class GemmReduceScatter:
 
     def __call__(self, a, b, out=None, stream=None):
         """``a [M, K_r]``, ``b [N, K_r]`` bf16 -> ``out [M / ranks, N]`` bf16 (this rank's rows of the sum)."""
+        if self._mc:
+            return self._in_switch(a, b, out, stream)
+        got = self._call(self.comm._h.value or 0, a, b, out, stream, self._workspace)
+        if got.__class__ is int:
+            raise MiniNcclError(got, "fused kernel on a failed communicator")
+        return got
+
+    def _in_switch(self, a, b, out, stream):
         import torch
 
         M, N = self.M, self.N
@@ -107,7 +117,7 @@ class GemmReduceScatter:
             out = torch.empty((M // self.comm.size, N), dtype=torch.bfloat16, device=a.device)
         s = stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream
         _check_comm(self.comm)
-        if self._mc and out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0:
+        if out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0:
             rc = _native().mncclGemmReduceScatterBf16Switch(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, a.shape[1],
                                                             a.stride(0), b.stride(0), out.stride(0), self.comm.rank,
                                                             self.comm.size, self._stage_peers, self._flag_peers,
@@ -143,6 +153,10 @@ class AllGatherGemm:
         self._ready = _peers(comm, self.ready)
         self._bar = _peers(comm, self.bar)
         self._handle = comm.device_handle_bytes()
+        self._handle_buf = C.create_string_buffer(self._handle, len(self._handle))
+        self._workspace = (M, K, comm.rank, R, C.addressof(self._xg), C.addressof(self._ready), C.addressof(self._bar),
+                           self.state.data_ptr(), C.addressof(self._handle_buf), len(self._handle))
+        self._call = ext().ag_gemm
 
     @property
     def local_shard(self):
@@ -155,27 +169,10 @@ class AllGatherGemm:
 
         ``swiglu=True``: the epilogue applies SwiGLU and ``out`` is ``[M, N_r / 2]``; the rows of ``b`` must then
         be interleaved in groups of 16 (:func:`interleave_gate_up`), N_r a multiple of 32."""
-        import torch
-
-        if b.dtype != torch.bfloat16 or b.shape[1] != self.K or b.stride(1) != 1:
-            raise TypeError("b must be bf16 [N, K] with a unit inner stride")
-        N = b.shape[0]
-        if swiglu and N % 32:
-            raise ValueError("SwiGLU in the epilogue needs N a multiple of 32")
-        n_out = N // 2 if swiglu else N
-        if out is None:
-            out = torch.empty((self.M, n_out), dtype=torch.bfloat16, device=b.device)
-        if tuple(out.shape) != (self.M, n_out) or out.dtype != torch.bfloat16 or out.stride(1) != 1:
-            raise ValueError(f"out must be bf16 [{self.M}, {n_out}] with a unit inner stride")
-        s = stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream
-        _check_comm(self.comm)
-        rc = _native().mncclAllGatherGemmBf16Comm(self._xg, b.data_ptr(), out.data_ptr(), self.M, N, self.K, self.K, b.stride(0),
-                                                  out.stride(0), self.comm.rank, self.comm.size, self._ready, self._bar,
-                                                  self.state.data_ptr(), self.n_comm, 1 if swiglu else 0, self._handle,
-                                                  len(self._handle), s)
-        if rc != 0:
-            raise RuntimeError(f"all-gather->GEMM kernel failed with code {rc}")
-        return out
+        got = self._call(self.comm._h.value or 0, self.n_comm, b, out, stream, swiglu, self._workspace)
+        if got.__class__ is int:
+            raise MiniNcclError(got, "fused kernel on a failed communicator")
+        return got
 
 
 def interleave_gate_up(w_gate, w_up):
