@@ -267,7 +267,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         uint32_t r[32];
 #pragma unroll
         for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(acc[i]);
-        epi.store(g, epoch, row, tn * kBN + c * 32, r, c, warp_smem, lane);
+        epi.store_piece(g, epoch, row, tn * kBN + c * 32, r, c, warp_smem, lane);
       }
       // the last reader leaves the counter clean for the next launch
       __syncwarp();

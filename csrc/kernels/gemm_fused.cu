@@ -159,6 +159,12 @@ struct RsEpilogue {
     __syncwarp();  // the scratch is reused by the next pair of pieces
   }
 
+  // (no split-K here: the tiles of this kernel are never cut)
+  __device__ __forceinline__ void store_piece(const GemmArgs& g, uint32_t epoch, int row, int col, const uint32_t (&r)[32],
+                                              int chunk, uint8_t* warp_smem, int lane) const {
+    store(g, epoch, row, col, r, chunk, warp_smem, lane);
+  }
+
   // All four epilogue warps call this after the last store of a tile.
   __device__ __forceinline__ void warp_begin(uint8_t*, int) const {}
 
@@ -183,8 +189,7 @@ struct RsEpilogue {
       reduce_switch<128, false>(g, epoch, ((q + 2) & 3) * 32 + lane, abort_flag);
       return;
     }
-    if (nranks <= 1) reduce_owned<1, 16>(g, epoch, cta, n_cta, q, lane, abort_flag);
-    else if (nranks <= 2) reduce_owned<2, 16>(g, epoch, cta, n_cta, q, lane, abort_flag);
+    if (nranks <= 2) reduce_owned<2, 16>(g, epoch, cta, n_cta, q, lane, abort_flag);
     else if (nranks <= 4) reduce_owned<4, 8>(g, epoch, cta, n_cta, q, lane, abort_flag);
     else reduce_owned<kMaxTpRanks, 4>(g, epoch, cta, n_cta, q, lane, abort_flag);
   }
@@ -333,59 +338,18 @@ struct AgEpilogue {
   uint32_t* bar[kMaxTpRanks];        // every rank's barrier words [n_comm][nranks] (unused since the done words)
   int done_base;                     // ready[r] + done_base + s: rank s has left its call number (value); see last_cta_out
   StoreEpilogue<false> plain;
-
-  int swiglu;                        // 1: the store applies SwiGLU (see store_swiglu); C is [M, N / 2]
-  int chunks_per_tile;               // 32-column pieces per tile (tile width / 32)
+  SwiGluEpilogue act;                // SwiGLU instead of the plain store where swiglu is set; C is [M, N / 2]
+  int swiglu;
 
   __device__ __forceinline__ void store(const GemmArgs& g, uint32_t epoch, int row, int col, const uint32_t (&r)[32],
                                         int chunk, uint8_t* warp_smem, int lane) const {
-    if (swiglu) store_swiglu(g, row, col, r, chunk, warp_smem, lane);
+    if (swiglu) act.store(g, epoch, row, col, r, chunk, warp_smem, lane);
     else plain.store(g, epoch, row, col, r, chunk, warp_smem, lane);
   }
-
-  // SwiGLU in the epilogue.  The weight's rows (the GEMM's columns) come interleaved in groups of 16:
-  // columns [32k, 32k+16) are gate features 16k.., columns [32k+16, 32k+32) the up features of the
-  // same indices, so one 32-column piece of an accumulator row holds both operands of 16 outputs:
-  //   act[row, 16k + j] = silu(acc[32k + j]) * acc[32k + 16 + j]        (fp32 math, one rounding)
-  // Up to four pieces (64 outputs = 128 bytes per row) are collected in shared memory and leave as
-  // whole rows, 8 lanes per row.  The H = (gate | up) matrix never reaches memory: the kernel
-  // writes half the bytes and the separate elementwise pass disappears.
-  __device__ __forceinline__ void store_swiglu(const GemmArgs& g, int row, int col, const uint32_t (&r)[32], int chunk,
-                                               uint8_t* warp_smem, int lane) const {
-    if (col >= g.N) return;  // the same for the whole warp (N is a multiple of 32 here)
-    const int part = chunk & 3;
-    uint8_t* mine = warp_smem + lane * kEpiRowBytes + part * 32;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      uint4 v;
-      uint32_t* w = reinterpret_cast<uint32_t*>(&v);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int i = 8 * j + 2 * k;
-        const float g0 = __uint_as_float(r[i]), g1 = __uint_as_float(r[i + 1]);
-        const float u0 = __uint_as_float(r[16 + i]), u1 = __uint_as_float(r[16 + i + 1]);
-        __nv_bfloat162 p = __floats2bfloat162_rn(g0 / (1.0f + __expf(-g0)) * u0, g1 / (1.0f + __expf(-g1)) * u1);
-        w[k] = *reinterpret_cast<uint32_t*>(&p);
-      }
-      *reinterpret_cast<uint4*>(mine + j * 16) = v;
-    }
-    const bool flush = part == 3 || chunk == chunks_per_tile - 1 || col + 32 >= g.N;
-    if (!flush) return;
-    __syncwarp();
-    const int row_base = row - lane;
-    const int out_col = (col - part * 32) / 2;       // first output column of the collected pieces
-    const int out_cols = (part + 1) * 16;
-    __nv_bfloat16* c = static_cast<__nv_bfloat16*>(g.c);
-#pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const int rr = it * 4 + (lane >> 3), seg = lane & 7;
-      const int grow = row_base + rr;
-      if (grow < g.M && seg * 8 < out_cols) {
-        const uint4 v = *reinterpret_cast<const uint4*>(warp_smem + rr * kEpiRowBytes + seg * 16);
-        *reinterpret_cast<uint4*>(c + static_cast<size_t>(grow) * g.ldc + out_col + seg * 8) = v;
-      }
-    }
-    __syncwarp();
+  __device__ __forceinline__ void store_piece(const GemmArgs& g, uint32_t epoch, int row, int col, const uint32_t (&r)[32],
+                                              int chunk, uint8_t* warp_smem, int lane) const {
+    if (swiglu) act.store_piece(g, epoch, row, col, r, chunk, warp_smem, lane);
+    else plain.store_piece(g, epoch, row, col, r, chunk, warp_smem, lane);
   }
   static constexpr int kWarpSmemBytes = kEpiWarpBytes;
   static constexpr int kSingleStages = kStages;
@@ -397,7 +361,6 @@ struct AgEpilogue {
   // The last CTA of the kernel (every tile done, every row of the gather buffer read): tell every peer
   // that this rank's gather buffer is free for the pushes of the next call.
   __device__ __forceinline__ void last_cta_out(const GemmArgs&, uint32_t epoch) const {
-    if (nranks <= 1 || ready[rank] == nullptr) return;
     __threadfence_system();
     for (int p = 0; p < nranks; ++p)
       if (p != rank) st_release_sys_u32(ready[p] + done_base + rank, epoch);
@@ -538,6 +501,10 @@ static int gemm_rs_launch(const void* A, const void* B, void* out, int M, int N,
   if (lda == 0) lda = K;
   if (ldb == 0) ldb = K;
   if (ldo == 0) ldo = N;
+  // One rank owns every row and adds nothing: the tile's one rounding to bf16 is the result, so the plain
+  // kernels store it where it belongs.  (Through the staging it was written, flagged, read back and
+  // written again: 4096 x 4096 x 1792 took 93 us where the product alone takes 39.)
+  if (nranks == 1) return run_gemm("GEMM->reduce-scatter", A, B, out, M, N, K, lda, ldb, ldo, kOutBf16, stream);
   CUtensorMap ta, tb;
   std::string why;
   // CTA pairs need every rank's rows to be whole 256-row tiles (the rasterisation works on pairs of m-tiles)
@@ -667,13 +634,16 @@ static int ag_gemm_launch(void* const* xg_peers, const void* B, void* C, int M, 
   if (lda == 0) lda = K;
   if (ldb == 0) ldb = K;
   if (ldc == 0) ldc = swiglu ? N / 2 : N;
+  // one rank: its rows are all there is, nothing to gather
+  if (nranks == 1)
+    return run_gemm("all-gather->GEMM", xg_peers[0], B, C, M, N, K, lda, ldb, ldc, swiglu ? kOutSwiGlu : kOutBf16, stream);
   CUtensorMap ta, tb;
   std::string why;
   // The A operand is this rank's own gather buffer: TMA only ever reads local memory.
-  const bool pair = ((M / nranks) % (2 * kBM)) == 0 && want_pair(M, N, sm_count() - (nranks > 1 ? 16 : 0)) &&
+  const bool pair = ((M / nranks) % (2 * kBM)) == 0 && want_pair(M, N, sm_count() - 16) &&
                     2 * max_pairs<AgEpilogue>() >= (sm_count() & ~1);
   // (the SwiGLU store collects pairs of 32-column pieces: no 224-wide tiles then)
-  const int bn = pair ? kBN : pick_tile_n(M, N, sm_count() - (nranks > 1 ? 16 : 0), !swiglu);
+  const int bn = pair ? kBN : pick_tile_n(M, N, sm_count() - 16, !swiglu);
   if (!make_tensor_map_bf16(&ta, xg_peers[rank], M, K, lda, kBM, kBK, &why) ||
       !make_tensor_map_bf16(&tb, B, N, K, ldb, pair ? kBN / 2 : bn, kBK, &why)) {
     fprintf(stderr, "[Mini-NCCL] all-gather->GEMM: %s\n", why.c_str());
@@ -681,34 +651,30 @@ static int ag_gemm_launch(void* const* xg_peers, const void* B, void* C, int M, 
   }
   const int sms = pair ? (sm_count() & ~1) : sm_count();
   const int all_tiles = (M / kBM) * ((N + bn - 1) / bn);
-  int n_comm = 0;
-  if (nranks > 1) {
-    if (n_comm_ctas > 0) {
-      n_comm = n_comm_ctas;
-    } else {
-      // The tiles need ceil(tiles / CTAs) waves anyway: give the GEMM just enough CTAs for that
-      // number of waves and let the rest move data (at least 16, at most 48).
-      const int waves = (all_tiles + (sms - 16) - 1) / (sms - 16);
-      const int need = (all_tiles + waves - 1) / waves;
-      n_comm = sms - need;
-      if (n_comm < 16) n_comm = 16;
-      if (n_comm > 48) n_comm = 48;
-    }
-    if (n_comm > sms / 2) n_comm = sms / 2;
-    if (pair) n_comm = (n_comm + 1) & ~1;  // communication CTAs come as whole clusters too
+  int n_comm = n_comm_ctas;
+  if (n_comm <= 0) {
+    // The tiles need ceil(tiles / CTAs) waves anyway: give the GEMM just enough CTAs for that
+    // number of waves and let the rest move data (at least 16, at most 48).
+    const int waves = (all_tiles + (sms - 16) - 1) / (sms - 16);
+    const int need = (all_tiles + waves - 1) / waves;
+    n_comm = sms - need;
+    if (n_comm < 16) n_comm = 16;
+    if (n_comm > 48) n_comm = 48;
   }
+  if (n_comm > sms / 2) n_comm = sms / 2;
+  if (pair) n_comm = (n_comm + 1) & ~1;  // communication CTAs come as whole clusters too
   AgEpilogue epi{};
   epi.rank = rank;
   epi.nranks = nranks;
   epi.rows_per_rank = M / nranks;
   epi.lda = lda;
   epi.swiglu = swiglu ? 1 : 0;
-  epi.chunks_per_tile = bn / 32;
+  epi.act.chunks_per_tile = bn / 32;
   epi.done_base = M / kBM;
   for (int r = 0; r < nranks; ++r) {
     epi.xg[r] = static_cast<char*>(xg_peers[r]);
-    epi.ready[r] = nranks > 1 ? static_cast<uint32_t*>(ready_peers[r]) : nullptr;
-    epi.bar[r] = nranks > 1 ? static_cast<uint32_t*>(bar_peers[r]) : nullptr;
+    epi.ready[r] = static_cast<uint32_t*>(ready_peers[r]);
+    epi.bar[r] = static_cast<uint32_t*>(bar_peers[r]);
   }
   GemmArgs g{};
   g.M = M;
@@ -725,13 +691,11 @@ static int ag_gemm_launch(void* const* xg_peers, const void* B, void* C, int M, 
   g.m_tile_rotate = rank * tiles_m_local;  // local rows first, then the shards in arrival order
   g.epoch_ptr = state;
   g.ticket_ptr = state + 1;
-  if (nranks > 1) {
-    g.a_ready = epi.ready[rank];
-    g.a_ready_mult = static_cast<uint32_t>(kAgPartsPerChunk);
-    g.rows_per_chunk = kBM;
-    g.a_local_first = rank * tiles_m_local;
-    g.a_local_count = tiles_m_local;
-  }
+  g.a_ready = epi.ready[rank];
+  g.a_ready_mult = static_cast<uint32_t>(kAgPartsPerChunk);
+  g.rows_per_chunk = kBM;
+  g.a_local_first = rank * tiles_m_local;
+  g.a_local_count = tiles_m_local;
   const int tiles = all_tiles;
   int n_gemm = sms - n_comm;
   if (tiles < n_gemm) n_gemm = tiles;

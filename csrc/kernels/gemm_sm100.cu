@@ -24,6 +24,7 @@
 #include <mutex>
 
 #include "kernels/gemm2_kernel.cuh"
+#include "kernels/gemm_small.h"
 #include "mem/cuda_driver.h"
 
 namespace mnccl {
@@ -43,8 +44,18 @@ int pair_mode_from_env() {
 }
 int g_use_pair = pair_mode_from_env();
 uint32_t* g_err_dev[kMaxDevices] = {};  // one error word per device of the process
-float* g_split_ws[kMaxDevices] = {};    // split-K workspace per device (fp32 partial tiles), allocated on first use
-uint32_t* g_split_cnt[kMaxDevices] = {};
+// Split-K workspaces: one per (device, stream) that has needed one, so that products on different streams do
+// not add into each other's partial tiles.  At most kSplitPools of them live (20 MB each, for the life of
+// the process); a stream beyond that computes without the split.
+struct SplitPool {
+  int dev;
+  cudaStream_t stream;
+  float* ws;       // fp32 partial tiles
+  uint32_t* cnt;   // one counter per 32-row quarter
+};
+constexpr int kSplitPools = 8;
+SplitPool g_split[kSplitPools];
+int g_split_used = 0;
 constexpr int kSplitMaxItems = 80;      // K-slices in flight: at most one per CTA pair
 
 }  // namespace
@@ -89,28 +100,35 @@ uint32_t* error_word() {
 }
 
 // Workspace of the split last wave: kSplitMaxItems partial tiles of 256 x 256 fp32 (20 MB) and one
-// counter per 32-row quarter.  Allocated once per device, the first time a shape is split (not under
-// stream capture: call the GEMM once before capturing).  Null when the allocation fails: no split then.
-bool split_workspace(float** ws, uint32_t** cnt) {
+// counter per 32-row quarter.  Allocated the first time a shape is split on `stream` (never under stream
+// capture: call the GEMM once on that stream before capturing).  False: no split then.
+bool split_workspace(cudaStream_t stream, float** ws, uint32_t** cnt) {
   std::lock_guard<std::mutex> lk(g_mu);
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= kMaxDevices) dev = 0;
-  if (g_split_ws[dev] == nullptr) {
-    float* w = nullptr;
-    uint32_t* c = nullptr;
-    if (cudaMalloc(&w, size_t(kSplitMaxItems) * 256 * 256 * 4) != cudaSuccess ||
-        cudaMalloc(&c, size_t(kSplitMaxItems) * 8 * 4) != cudaSuccess) {
-      (void)cudaGetLastError();
-      if (w) cudaFree(w);
-      return false;
+  const int dev = current_device_slot();
+  for (int i = 0; i < g_split_used; ++i) {
+    if (g_split[i].dev == dev && g_split[i].stream == stream) {
+      *ws = g_split[i].ws;
+      *cnt = g_split[i].cnt;
+      return true;
     }
-    cudaMemset(c, 0, size_t(kSplitMaxItems) * 8 * 4);
-    g_split_ws[dev] = w;
-    g_split_cnt[dev] = c;
   }
-  *ws = g_split_ws[dev];
-  *cnt = g_split_cnt[dev];
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (g_split_used == kSplitPools || cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return false;
+  }
+  SplitPool p{dev, stream, nullptr, nullptr};
+  if (cudaMalloc(&p.ws, size_t(kSplitMaxItems) * 256 * 256 * 4) != cudaSuccess ||
+      cudaMalloc(&p.cnt, size_t(kSplitMaxItems) * 8 * 4) != cudaSuccess ||
+      cudaMemset(p.cnt, 0, size_t(kSplitMaxItems) * 8 * 4) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    (void)cudaGetLastError();
+    if (p.ws) cudaFree(p.ws);
+    if (p.cnt) cudaFree(p.cnt);
+    return false;
+  }
+  g_split[g_split_used++] = p;
+  *ws = p.ws;
+  *cnt = p.cnt;
   return true;
 }
 
@@ -191,6 +209,133 @@ int sm_count() {
   return sms;
 }
 
+namespace {
+
+// Estimated times (ns) on this GPU's 148 SMs, measured for square-ish and for thin products with K from 64 to
+// 14336 (graph replay, operands not in L2).  They only have to rank the candidates.
+//
+// Small kernel (gemm_small.cu), tiles of 128 rows of B x tn rows of A, K over `slices` CTAs: a fixed part
+// (launch, first loads, epilogue, meeting of the slices), a time per k-block and SM, which is what L2 can
+// hand one SM, and never faster than DRAM delivers the operands.
+struct SmallCost {
+  int tn, kps;              // rows of A per tile, k-blocks per stage
+  long fixed, fixed_split;  // one slice, several slices
+  long per_kb;
+};
+constexpr SmallCost kSmallCost[] = {{16, 2, 3500, 4500, 130}, {32, 2, 4100, 4900, 145}, {64, 2, 4400, 5000, 173}, {128, 1, 5900, 6300, 240}};
+
+long dram_ns(int M, int N, int K, int out_bytes) {
+  return static_cast<long>((2.0 * K * (static_cast<double>(M) + N) + static_cast<double>(out_bytes) * M * N) / 6200.0);
+}
+
+long plan_small(int M, int N, int K, int out_bytes, int sms, SmallPlan* best) {
+  const int num_kb = (K + kBK - 1) / kBK;
+  const long tiles_n = (N + 127) / 128, floor_ns = 3000 + dram_ns(M, N, K, out_bytes);
+  long best_ns = -1;
+  for (const SmallCost& c : kSmallCost) {
+    if (c.tn > 16 && c.tn / 2 >= M) break;  // half of the tile would be padding
+    const long tiles = tiles_n * ((M + c.tn - 1) / c.tn);
+    if (tiles > 4L * sms) continue;
+    const int stages = (num_kb + c.kps - 1) / c.kps;
+    for (int s = 1; s <= 8; s *= 2) {
+      const int per = (stages + s - 1) / s;
+      if ((s - 1) * per >= stages) break;  // a slice would be empty
+      const long items = tiles * s;
+      if (s > 1 && items > 2L * sms) break;
+      // One CTA per SM where all of them fit at once (clusters of 4 and 8 do not tile every GPC: 15 clusters of
+      // 8 start together, a 16th waits for a whole round); else two share an SM and its L2 port.
+      const bool deep = items <= (s == 8 ? 15 * sms / 18 : s == 4 ? 7 * sms / 8 : sms);
+      const long rounds = deep ? 1 : 2 * ((items + 2L * sms - 1) / (2L * sms));
+      const long fixed = s == 1 ? c.fixed : s == 8 ? c.fixed_split + 1300 : c.fixed_split;
+      const long ns = std::max(fixed + rounds * per * c.kps * c.per_kb, floor_ns);
+      if (best_ns < 0 || ns < best_ns) {
+        best_ns = ns;
+        best->tn = c.tn;
+        best->slices = s;
+        best->kb_per_slice = per;
+        best->tiles = static_cast<int>(tiles);
+        best->deep = deep;
+      }
+    }
+  }
+  return best_ns;
+}
+
+// Persistent kernels: waves of tiles, a k-block of a 256 x 256 pair tile in 330 ns, of a 128 x bn tile at what L2
+// hands one SM (165 bytes per ns) or, narrow ones, at a quarter of the latency that the four-stage ring covers.
+long persistent_ns(int M, int N, int K, int out_bytes, int sms, bool pair, int bn) {
+  const long num_kb = (K + kBK - 1) / kBK;
+  const long floor_ns = 5000 + dram_ns(M, N, K, out_bytes);
+  if (pair) {
+    const long tiles = static_cast<long>((M + 2 * kBM - 1) / (2 * kBM)) * ((N + kBN - 1) / kBN);
+    const long waves = (tiles + sms / 2 - 1) / (sms / 2);
+    return std::max(5600 + waves * num_kb * 330, floor_ns);
+  }
+  const long tiles = static_cast<long>((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
+  const long waves = (tiles + sms - 1) / sms;
+  return std::max(4800 + waves * num_kb * std::max((kBM + bn) * 128 / 165, 285), floor_ns);
+}
+
+}  // namespace
+
+int run_gemm(const char* who, const void* A, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc, GemmOut out,
+             cudaStream_t stream) {
+  const int sms = sm_count();
+  const int out_bytes = out == kOutF32 ? 4 : 2;
+  const bool pair = want_pair(M, N, sms);
+  const int bn = pair ? kBN : pick_tile_n(M, N, sms, out != kOutSwiGlu);  // (the SwiGLU store collects whole rows of 32-column pieces)
+  std::string why;
+  if (g_use_pair < 0) {
+    // Small products, in automatic mode only: a pinned choice names one of the persistent kernels.
+    SmallPlan p;
+    const long small_ns = plan_small(M, N, K, out_bytes, sms, &p);
+    if (small_ns > 0 && small_ns < persistent_ns(M, N, K, out_bytes, sms, pair, bn)) {
+      const cudaError_t e = launch_small(A, B, C, M, N, K, lda, ldb, ldc, static_cast<int>(out), p, error_word(), stream, &why);
+      if (!why.empty()) {
+        fprintf(stderr, "[Mini-NCCL] %s: %s\n", who, why.c_str());
+        return -3;
+      }
+      return e == cudaSuccess ? 0 : static_cast<int>(e) + 1000;
+    }
+  }
+  CUtensorMap ta, tb;
+  // CTA pairs: 256 x 256 tiles, each CTA loads 128 rows of A and 128 rows (half of N) of B
+  if (!make_tensor_map_bf16(&ta, A, M, K, lda, kBM, kBK, &why) ||
+      !make_tensor_map_bf16(&tb, B, N, K, ldb, pair ? kBN / 2 : bn, kBK, &why)) {
+    fprintf(stderr, "[Mini-NCCL] %s: %s\n", who, why.c_str());
+    return -3;
+  }
+  GemmArgs g{};
+  g.M = M;
+  g.N = N;
+  g.K = K;
+  g.c = C;
+  g.ldc = ldc;
+  g.err = error_word();
+  g.wait_budget_ns = 2000000000ull;
+  g.group_m = 8;
+  int grid;
+  if (pair) {
+    const int tiles2 = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + kBN - 1) / kBN);
+    grid = std::min(2 * tiles2, sms & ~1);
+    const int pairs = std::min(grid / 2, out == kOutSwiGlu ? max_pairs<SwiGluEpilogue>() : max_pairs<StoreEpilogue<false>>());
+    int first = 0, slices = 0, per = 0;
+    if (plan_split(tiles2, pairs, (K + kBK - 1) / kBK, &first, &slices, &per) && split_workspace(stream, &g.split_ws, &g.split_cnt)) {
+      g.split_first = first;
+      g.split_s = slices;
+      g.split_kb = per;
+    }
+  } else {
+    grid = std::min(((M + kBM - 1) / kBM) * ((N + bn - 1) / bn), sms);
+  }
+  const auto fire = [&](const auto& epi) { return pair ? launch_pair(ta, tb, g, epi, grid, stream) : launch(ta, tb, g, epi, grid, stream, bn); };
+  cudaError_t e;
+  if (out == kOutF32) e = fire(StoreEpilogue<true>{});
+  else if (out == kOutSwiGlu) e = fire(SwiGluEpilogue{bn / 32});
+  else e = fire(StoreEpilogue<false>{});
+  return e == cudaSuccess ? 0 : static_cast<int>(e) + 1000;
+}
+
 }  // namespace gemm
 }  // namespace mnccl
 
@@ -212,47 +357,7 @@ MNCCL_EXPORT int mncclGemmBf16(const void* A, const void* B, void* C, int M, int
   if (ldb == 0) ldb = K;
   if (ldc == 0) ldc = N;
   if (lda < K || ldb < K || ldc < N) return -2;
-  CUtensorMap ta, tb;
-  std::string why;
-  GemmArgs g{};
-  g.M = M;
-  g.N = N;
-  g.K = K;
-  g.c = C;
-  g.ldc = ldc;
-  g.err = error_word();
-  g.wait_budget_ns = 2000000000ull;
-  g.group_m = 8;
-  cudaError_t e;
-  const bool pair = want_pair(M, N, sm_count());
-  if (pair) {
-    // CTA pairs: 256 x 256 tiles, each CTA loads 128 rows of A and 128 rows (half of N) of B
-    if (!make_tensor_map_bf16(&ta, A, M, K, lda, kBM, kBK, &why) || !make_tensor_map_bf16(&tb, B, N, K, ldb, kBN / 2, kBK, &why)) {
-      fprintf(stderr, "[Mini-NCCL] GEMM: %s\n", why.c_str());
-      return -3;
-    }
-    const int tiles2 = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + kBN - 1) / kBN);
-    int grid = 2 * tiles2;
-    if (grid > (sm_count() & ~1)) grid = sm_count() & ~1;
-    const int pairs = std::min(grid / 2, max_pairs<StoreEpilogue<false>>());
-    int first = 0, slices = 0, per = 0;
-    if (plan_split(tiles2, pairs, (K + kBK - 1) / kBK, &first, &slices, &per) && split_workspace(&g.split_ws, &g.split_cnt)) {
-      g.split_first = first;
-      g.split_s = slices;
-      g.split_kb = per;
-    }
-    e = out_f32 ? launch_pair(ta, tb, g, StoreEpilogue<true>{}, grid, stream) : launch_pair(ta, tb, g, StoreEpilogue<false>{}, grid, stream);
-  } else {
-    const int bn = pick_tile_n(M, N, sm_count(), true);
-    if (!make_tensor_map_bf16(&ta, A, M, K, lda, kBM, kBK, &why) || !make_tensor_map_bf16(&tb, B, N, K, ldb, bn, kBK, &why)) {
-      fprintf(stderr, "[Mini-NCCL] GEMM: %s\n", why.c_str());
-      return -3;
-    }
-    const int tiles = ((M + kBM - 1) / kBM) * ((N + bn - 1) / bn);
-    const int grid = tiles < sm_count() ? tiles : sm_count();
-    e = out_f32 ? launch(ta, tb, g, StoreEpilogue<true>{}, grid, stream, bn) : launch(ta, tb, g, StoreEpilogue<false>{}, grid, stream, bn);
-  }
-  return e == cudaSuccess ? 0 : static_cast<int>(e) + 1000;
+  return run_gemm("GEMM", A, B, C, M, N, K, lda, ldb, ldc, out_f32 ? kOutF32 : kOutBf16, stream);
 }
 
 // Pairs of CTAs (clusters of 2) of the GEMM kernel that fit the current device at once.
@@ -267,6 +372,22 @@ MNCCL_EXPORT void mncclGemmSetPairMode(int mode) { set_pair_mode(mode); }
 MNCCL_EXPORT void mncclGemmPlan(int M, int N, int ctas, int narrow, int* tile_n, int* pair) {
   if (tile_n) *tile_n = pick_tile_n(M, N, ctas, narrow != 0);
   if (pair) *pair = want_pair(M, N, ctas) ? 1 : 0;
+}
+
+// Whether an M x N x K product (out: 0 bf16, 1 fp32, 2 SwiGLU) takes the kernel for small products on `sms` SMs in
+// automatic mode, and its plan: rows of A per tile, CTAs that share a tile's K, one CTA per SM or two.  Host
+// arithmetic only (needs no GPU).
+MNCCL_EXPORT int mncclGemmSmallPlan(int M, int N, int K, int out, int sms, int* tn, int* slices, int* deep) {
+  if (M <= 0 || N <= 0 || K <= 0 || sms <= 0) return 0;
+  SmallPlan p;
+  const bool pair = want_pair(M, N, sms);
+  const int bn = pair ? kBN : pick_tile_n(M, N, sms, out != kOutSwiGlu), out_bytes = out == kOutF32 ? 4 : 2;
+  const long ns = plan_small(M, N, K, out_bytes, sms, &p);
+  if (ns < 0 || ns >= persistent_ns(M, N, K, out_bytes, sms, pair, bn)) return 0;
+  if (tn) *tn = p.tn;
+  if (slices) *slices = p.slices;
+  if (deep) *deep = p.deep ? 1 : 0;
+  return 1;
 }
 
 // The split-K plan of the CTA-pair kernel for an M x N x K product on `pairs` CTA pairs, without launching
