@@ -81,6 +81,18 @@ int mncclAllGatherGemmBf16(void* const* xg_peers, const void* B, void* C, int M,
  * F, ldh, lda multiples of 8; both pointers 16-byte aligned. */
 int mncclSwiGluBf16(const void* h, void* act, int M, int F, long ldh, long lda, cudaStream_t stream);
 
+/* ---- cross-entropy of a language-model head ---------------------------------------------------------
+ * Mean cross-entropy of bf16 logits [T, V] against T class indices (-100: the row counts for nothing), fp32 math.
+ * Rows are 16-byte aligned and their stride, in elements, is a multiple of 8 that holds the row rounded up to one.
+ * Forward: picked[t] = logit of row t's target; writes lse[T], row_loss[T] (scratch) and mean[2] = {loss, rows
+ * that count}.  Backward: gradient times grad[0], as d [T, V] and / or dt [V, T] (either may be null). */
+int mncclLmLossForward(const void* logits, int64_t ld, int T, int V, const int64_t* targets, const void* picked, float* lse,
+                       float* row_loss, float* mean, cudaStream_t stream);
+int mncclLmLossBackward(const void* logits, int64_t ld, int T, int V, const int64_t* targets, const float* lse, const float* grad,
+                        const float* mean, void* d, int64_t ldd, void* dt, int64_t ldt, cudaStream_t stream);
+/* dst[cols, rows] = src[rows, cols]^T, bf16, rows laid out as above. */
+int mncclTransposeBf16(const void* src, int64_t lds, int rows, int cols, void* dst, int64_t ldd, cudaStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -102,6 +102,10 @@ def lib() -> C.CDLL:
             sig("mncclGemmPlan", None, i32, i32, i32, i32, C.POINTER(C.c_int), C.POINTER(C.c_int))
     if hasattr(L, "mncclSwiGluBf16"):
         sig("mncclSwiGluBf16", i32, vp, vp, i32, i32, C.c_long, C.c_long, vp)
+    if hasattr(L, "mncclLmLossForward"):
+        sig("mncclLmLossForward", i32, vp, C.c_int64, i32, i32, vp, vp, vp, vp, vp, vp)
+        sig("mncclLmLossBackward", i32, vp, C.c_int64, i32, i32, vp, vp, vp, vp, vp, C.c_int64, vp, C.c_int64, vp)
+        sig("mncclTransposeBf16", i32, vp, C.c_int64, i32, i32, vp, C.c_int64, vp)
     if hasattr(L, "mncclGemmReduceScatterBf16"):
         sig("mncclGemmRsStageBytes", sz, i32, i32, i32)
         sig("mncclGemmRsFlagWords", sz, i32, i32, i32)

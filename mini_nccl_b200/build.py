@@ -49,7 +49,7 @@ CUDA_SOURCES = [
     "kernels/launch.cu", "emu/emu_world.cu",
 ]
 # Translation units compiled when present (a source tree may be trimmed to the collectives alone).
-OPTIONAL_CUDA = ["kernels/gemm_sm100.cu", "kernels/gemm_small.cu", "kernels/gemm_fused.cu", "kernels/noalloc.cu", "kernels/elementwise.cu"]
+OPTIONAL_CUDA = ["kernels/gemm_sm100.cu", "kernels/gemm_small.cu", "kernels/gemm_fused.cu", "kernels/noalloc.cu", "kernels/elementwise.cu", "kernels/lm_loss.cu"]
 OPTIONAL_HOST = ["net/verbs_transport.cc"]
 
 _HERA_SRCS = ["csrc/bootstrap/hera.cc", "csrc/bootstrap/socket.cc", "csrc/core/log.cc"]

@@ -2,9 +2,9 @@
 
 The reference has no model code; this is the synthetic workload the DDP
 configuration names: 24 layers, d_model 1024, 16 heads, vocabulary 50257,
-sequence 1024, bf16 weights, random initialisation.  Compute runs on PyTorch's
-library kernels (the communication library is the product under test here); the
-gradient AllReduce goes through mini_nccl_b200.parallel.ddp.
+sequence 1024, bf16 weights, random initialisation.  The output projection and
+the loss run on this library's kernels (ops/lm_loss.py), the rest of the compute
+on PyTorch's; the gradient AllReduce goes through mini_nccl_b200.parallel.ddp.
 """
 from __future__ import annotations
 
@@ -13,6 +13,8 @@ from dataclasses import dataclass
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+
+from ..ops.lm_loss import lm_head_cross_entropy
 
 
 @dataclass
@@ -76,10 +78,10 @@ class GPT2Model(nn.Module):
         x = self.wte(ids) + self.wpe(pos)
         for blk in self.blocks:
             x = blk(x)
-        logits = F.linear(self.ln_f(x), self.wte.weight)  # tied output embedding
+        x = self.ln_f(x)
         if targets is None:
-            return logits
-        return F.cross_entropy(logits.float().view(-1, logits.size(-1)), targets.view(-1))
+            return F.linear(x, self.wte.weight)  # tied output embedding
+        return lm_head_cross_entropy(x, self.wte.weight, targets)
 
     def num_params(self) -> int:
         return sum(p.numel() for p in self.parameters())

@@ -3,3 +3,4 @@ with the collectives (GEMM -> reduce-scatter, all-gather -> GEMM)."""
 from .gemm import gemm_bf16, gemm_status  # noqa: F401
 from .fused import AllGatherGemm, GemmReduceScatter, interleave_gate_up, split_gate_up  # noqa: F401,E402
 from .elementwise import swiglu_bf16  # noqa: F401,E402
+from .lm_loss import lm_head_cross_entropy  # noqa: F401,E402
