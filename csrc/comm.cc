@@ -16,6 +16,7 @@
 #include "bootstrap/fdpass.h"
 #include "bootstrap/hera.h"
 #include "bootstrap/store.h"
+#include "core/graph_capture.h"
 #include "core/log.h"
 #include "core/nvtx.h"
 #include "mem/cuda_driver.h"
@@ -572,17 +573,10 @@ Comm::~Comm() {
       cudaEventDestroy(pipe_->ev_comm[h]);
       cudaEventDestroy(pipe_->ev_out[h]);
     }
-    for (int h = 0; h < kSoloSlots; ++h) {
-      if (pipe_->ev_filled[h]) cudaEventDestroy(pipe_->ev_filled[h]);
-      if (pipe_->ev_work[h]) cudaEventDestroy(pipe_->ev_work[h]);
-      if (pipe_->ev_done[h]) cudaEventDestroy(pipe_->ev_done[h]);
-    }
     pipe_.reset();
   }
-  if (solo_stage_) {
-    cudaFree(solo_stage_);
-    solo_stage_ = nullptr;
-  }
+  solo_ring_.destroy();
+  for (auto& r : solo_graph_rings_) r->destroy();
   for (int r = 0; r < static_cast<int>(shared_peer_stage_.size()); ++r)
     if (r != rank_ && shared_peer_stage_[r]) cudaIpcCloseMemHandle(shared_peer_stage_[r]);
   shared_peer_stage_.clear();
@@ -826,11 +820,6 @@ void Comm::ensure_pipeline() {
       RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_comm[h], cudaEventDisableTiming), "cudaEventCreate");
       RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_out[h], cudaEventDisableTiming), "cudaEventCreate");
     }
-    for (int h = 0; size_ == 1 && h < kSoloSlots; ++h) {
-      RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_filled[h], cudaEventDisableTiming), "cudaEventCreate");
-      RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_work[h], cudaEventDisableTiming), "cudaEventCreate");
-      RT_CHECK(cudaEventCreateWithFlags(&pipe_->ev_done[h], cudaEventDisableTiming), "cudaEventCreate");
-    }
   }
 }
 
@@ -974,17 +963,11 @@ void Comm::solo_all_reduce(const void* send, DType send_t, void* recv, DType rec
   stats_.bytes += in_bytes;
   const bool in_place = send == recv && send_t == recv_t && la.identity;  // nothing to do
   if ((host_in || host_out) && !in_place) {
-    // The first pipelined call creates streams, events and device staging: not while a graph is being
-    // captured.  Such a call takes the kernel instead.
     const size_t bytes = std::max(in_bytes, out_bytes);
-    bool pipeline = cfg_.host_pipeline_min_bytes != 0 && bytes >= std::max(cfg_.host_pipeline_min_bytes, 2 * cfg_.host_chunk_bytes);
-    if (pipeline && (!pipe_ || solo_slot_bytes_ < solo_chunk_bytes(SIZE_MAX))) {
-      cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-      if (cudaStreamIsCapturing(stream, &cs) != cudaSuccess) (void)cudaGetLastError();
-      if (cs == cudaStreamCaptureStatusActive) pipeline = false;
-    }
-    if (pipeline) {
-      launch_solo_host(la, send_t, recv_t, stream, host_in, host_out);
+    const bool pipeline = cfg_.host_pipeline_min_bytes != 0 && bytes >= std::max(cfg_.host_pipeline_min_bytes, 2 * cfg_.host_chunk_bytes);
+    SoloRing* ring = pipeline ? solo_ring(stream) : nullptr;
+    if (ring != nullptr) {
+      launch_solo_host(*ring, la, send_t, recv_t, stream, host_in, host_out);
       stats_.pipelined++;
       return;
     }
@@ -1002,33 +985,90 @@ size_t Comm::solo_chunk_bytes(size_t bytes) const {
   return std::max<size_t>((c + 65535) & ~size_t(65535), 65536);
 }
 
+void Comm::SoloRing::destroy() {
+  if (s_in) cudaStreamDestroy(s_in);
+  if (s_out) cudaStreamDestroy(s_out);
+  const auto drop = [](cudaEvent_t& e) {
+    if (e) cudaEventDestroy(e);
+    e = nullptr;
+  };
+  drop(ev_start);
+  drop(ev_last);
+  for (int h = 0; h < kSoloSlots; ++h) {
+    drop(ev_filled[h]);
+    drop(ev_work[h]);
+    drop(ev_done[h]);
+  }
+  if (stage) cudaFree(stage);
+  s_in = s_out = nullptr;
+  stage = nullptr;
+}
+
+void Comm::create_ring(SoloRing& r) {
+  AllowAllocationsWhileCapturing allow;
+  const auto event = [](cudaEvent_t& e) {
+    if (e == nullptr) RT_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+  };
+  if (r.s_in == nullptr) RT_CHECK(cudaStreamCreateWithFlags(&r.s_in, cudaStreamNonBlocking), "cudaStreamCreate");
+  if (r.s_out == nullptr) RT_CHECK(cudaStreamCreateWithFlags(&r.s_out, cudaStreamNonBlocking), "cudaStreamCreate");
+  event(r.ev_start);
+  event(r.ev_last);
+  for (int h = 0; h < kSoloSlots; ++h) {
+    event(r.ev_filled[h]);
+    event(r.ev_work[h]);
+    event(r.ev_done[h]);
+  }
+  if (r.stage == nullptr) {
+    // slots for the largest chunk, so that a ring never has to grow
+    r.slot_bytes = solo_chunk_bytes(SIZE_MAX);
+    RT_CHECK(cudaMalloc(reinterpret_cast<void**>(&r.stage), kSoloSlots * r.slot_bytes), "cudaMalloc (host staging)");
+  }
+}
+
+// The ring for a call on `stream`; null for a captured call that finds none left.
+Comm::SoloRing* Comm::solo_ring(cudaStream_t stream) {
+  const CaptureInfo cap = capture_info(stream);
+  if (!cap.active) {
+    create_ring(solo_ring_);
+    return &solo_ring_;
+  }
+  // Calls of one capture on one stream run one after the other, in every replay: they share a ring.
+  SoloRing* idle = nullptr;
+  for (auto& r : solo_graph_rings_) {
+    if (!r->in_graph->load(std::memory_order_acquire)) idle = r.get();
+    else if (r->capture_id == cap.id && r->capture_stream == stream) return r.get();
+  }
+  if (idle == nullptr) {
+    if (solo_graph_rings_.size() == kSoloGraphRings) return nullptr;
+    solo_graph_rings_.emplace_back(new SoloRing());
+    idle = solo_graph_rings_.back().get();
+    idle->in_graph = std::make_shared<std::atomic<bool>>(false);
+  }
+  create_ring(*idle);
+  if (!hold_while_graph_lives(cap.graph, idle->in_graph)) return nullptr;
+  idle->capture_id = cap.id;
+  idle->capture_stream = stream;
+  return idle;
+}
+
 // One rank, pinned host buffers, as a pipeline through a ring of device slots: copy engine in, kernel (only
 // where something is scaled or converted), copy engine out.  Host -> device and device -> host run at the
 // same time (PCIe is full duplex).
-void Comm::launch_solo_host(const LocalArgs& call, DType send_t, DType recv_t, cudaStream_t stream, bool host_in, bool host_out) {
-  ensure_pipeline();
+void Comm::launch_solo_host(SoloRing& r, const LocalArgs& call, DType send_t, DType recv_t, cudaStream_t stream, bool host_in,
+                            bool host_out) {
   const size_t isz = dtype_size(send_t), osz = dtype_size(recv_t), wide = std::max(isz, osz);
-  // Slots for the largest chunk from the start: a captured call keeps their addresses.
-  const size_t slot = solo_chunk_bytes(SIZE_MAX);
-  if (solo_stage_ == nullptr || solo_slot_bytes_ < slot) {
-    if (solo_stage_) {
-      RT_CHECK(cudaDeviceSynchronize(), "cudaDeviceSynchronize");
-      cudaFree(solo_stage_);
-      solo_stage_ = nullptr;
-      solo_slot_bytes_ = 0;
-    }
-    RT_CHECK(cudaMalloc(reinterpret_cast<void**>(&solo_stage_), kSoloSlots * slot), "cudaMalloc (host staging)");
-    solo_slot_bytes_ = slot;
-  }
   const size_t chunk = solo_chunk_bytes(call.count * wide) / wide;
   const bool kernel = !(send_t == recv_t && call.identity);
   // slots: all of them hold input on its way to the output, or half of them inputs and half results
   const int ring = kernel ? kSoloSlots / 2 : kSoloSlots;
-  char* const out_slots = solo_stage_ + (kernel ? ring * solo_slot_bytes_ : 0);
+  char* const out_slots = r.stage + (kernel ? ring * r.slot_bytes : 0);
+  // The call before this one may have run on another stream: its last use of the ring comes first.  (No cost on
+  // one stream.  An event that was never recorded is waited for by nobody.)
+  if (&r == &solo_ring_) RT_CHECK(cudaStreamWaitEvent(stream, r.ev_last, 0), "cudaStreamWaitEvent");
   // only the side streams that get work are forked (a forked stream must be joined under capture)
-  RT_CHECK(cudaEventRecord(pipe_->ev_start, stream), "cudaEventRecord");
-  if (host_in) RT_CHECK(cudaStreamWaitEvent(pipe_->s_in, pipe_->ev_start, 0), "cudaStreamWaitEvent");
-  if (host_out) RT_CHECK(cudaStreamWaitEvent(pipe_->s_out, pipe_->ev_start, 0), "cudaStreamWaitEvent");
+  RT_CHECK(cudaEventRecord(r.ev_start, stream), "cudaEventRecord");
+  if (host_in) RT_CHECK(cudaStreamWaitEvent(r.s_in, r.ev_start, 0), "cudaStreamWaitEvent");
+  if (host_out) RT_CHECK(cudaStreamWaitEvent(r.s_out, r.ev_start, 0), "cudaStreamWaitEvent");
   int i = 0;
   for (size_t off = 0; off < call.count; off += chunk, ++i) {
     const int h = i % ring;
@@ -1036,42 +1076,40 @@ void Comm::launch_solo_host(const LocalArgs& call, DType send_t, DType recv_t, c
     const char* src = static_cast<const char*>(call.send) + off * isz;
     char* dst = static_cast<char*>(call.recv) + off * osz;
     const char* k_in = src;      // what the kernel (or the copy out) reads
-    cudaStream_t last = stream;  // where the result of this chunk is produced
     if (host_in) {
-      char* a_h = (!kernel && !host_out) ? dst : solo_stage_ + h * solo_slot_bytes_;   // host -> device, nothing to convert: straight in
+      char* a_h = (!kernel && !host_out) ? dst : r.stage + h * r.slot_bytes;   // host -> device, nothing to convert: straight in
       // the slot's last reader: the kernel, or the copy out of a pipeline without one
       if (i >= ring && (kernel || host_out))
-        RT_CHECK(cudaStreamWaitEvent(pipe_->s_in, kernel ? pipe_->ev_work[h] : pipe_->ev_done[h], 0), "cudaStreamWaitEvent");
-      RT_CHECK(cudaMemcpyAsync(a_h, src, n * isz, cudaMemcpyHostToDevice, pipe_->s_in), "cudaMemcpyAsync");
-      RT_CHECK(cudaEventRecord(pipe_->ev_filled[h], pipe_->s_in), "cudaEventRecord");
+        RT_CHECK(cudaStreamWaitEvent(r.s_in, kernel ? r.ev_work[h] : r.ev_done[h], 0), "cudaStreamWaitEvent");
+      RT_CHECK(cudaMemcpyAsync(a_h, src, n * isz, cudaMemcpyHostToDevice, r.s_in), "cudaMemcpyAsync");
+      RT_CHECK(cudaEventRecord(r.ev_filled[h], r.s_in), "cudaEventRecord");
       k_in = a_h;
-      last = pipe_->s_in;
     }
     if (kernel) {
-      char* b_h = host_out ? out_slots + h * solo_slot_bytes_ : dst;
-      if (host_in) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_filled[h], 0), "cudaStreamWaitEvent");
-      if (host_out && i >= ring) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_done[h], 0), "cudaStreamWaitEvent");
+      char* b_h = host_out ? out_slots + h * r.slot_bytes : dst;
+      if (host_in) RT_CHECK(cudaStreamWaitEvent(stream, r.ev_filled[h], 0), "cudaStreamWaitEvent");
+      if (host_out && i >= ring) RT_CHECK(cudaStreamWaitEvent(stream, r.ev_done[h], 0), "cudaStreamWaitEvent");
       LocalArgs la = call;
       la.send = k_in;
       la.recv = b_h;
       la.count = n;
       RT_CHECK(launch_local(send_t, recv_t, la, 0, stream), "kernel launch");
-      RT_CHECK(cudaEventRecord(pipe_->ev_work[h], stream), "cudaEventRecord");
+      RT_CHECK(cudaEventRecord(r.ev_work[h], stream), "cudaEventRecord");
       k_in = b_h;
-      last = stream;
     }
     if (host_out) {
-      if (last != stream || kernel)
-        RT_CHECK(cudaStreamWaitEvent(pipe_->s_out, kernel ? pipe_->ev_work[h] : pipe_->ev_filled[h], 0), "cudaStreamWaitEvent");
-      RT_CHECK(cudaMemcpyAsync(dst, k_in, n * osz, cudaMemcpyDeviceToHost, pipe_->s_out), "cudaMemcpyAsync");
-      RT_CHECK(cudaEventRecord(pipe_->ev_done[h], pipe_->s_out), "cudaEventRecord");
+      if (host_in || kernel)
+        RT_CHECK(cudaStreamWaitEvent(r.s_out, kernel ? r.ev_work[h] : r.ev_filled[h], 0), "cudaStreamWaitEvent");
+      RT_CHECK(cudaMemcpyAsync(dst, k_in, n * osz, cudaMemcpyDeviceToHost, r.s_out), "cudaMemcpyAsync");
+      RT_CHECK(cudaEventRecord(r.ev_done[h], r.s_out), "cudaEventRecord");
     }
   }
   stats_.by_algo[static_cast<int>(Algo::Local)]++;
   // the side streams run in order: their last event stands for all of their work
   const int h = (i - 1) % ring;
-  if (host_out) RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_done[h], 0), "cudaStreamWaitEvent");
-  else RT_CHECK(cudaStreamWaitEvent(stream, pipe_->ev_filled[h], 0), "cudaStreamWaitEvent");
+  if (host_out) RT_CHECK(cudaStreamWaitEvent(stream, r.ev_done[h], 0), "cudaStreamWaitEvent");
+  else RT_CHECK(cudaStreamWaitEvent(stream, r.ev_filled[h], 0), "cudaStreamWaitEvent");
+  if (&r == &solo_ring_) RT_CHECK(cudaEventRecord(r.ev_last, stream), "cudaEventRecord");
 }
 
 void Comm::wait_blocking(cudaStream_t stream) {

@@ -91,7 +91,11 @@ class Comm {
                         double scale, Algo forced, cudaStream_t stream, bool host_in = false, bool host_out = false);
   void solo_all_reduce(const void* send, DType send_t, void* recv, DType recv_t, DType wire_t, size_t count, RedOp op,
                        double scale, cudaStream_t stream);
-  void launch_solo_host(const LocalArgs& call, DType send_t, DType recv_t, cudaStream_t stream, bool host_in, bool host_out);
+  struct SoloRing;
+  void launch_solo_host(SoloRing& ring, const LocalArgs& call, DType send_t, DType recv_t, cudaStream_t stream, bool host_in,
+                        bool host_out);
+  SoloRing* solo_ring(cudaStream_t stream);
+  void create_ring(SoloRing& r);
   size_t solo_chunk_bytes(size_t bytes) const;
   void ensure_pipeline();
   void ring_all_reduce(const void* send, void* recv, size_t count, DType t, RedOp op, cudaStream_t stream);
@@ -151,16 +155,30 @@ class Comm {
   void auto_import();                        // map what the peers have exported since the last look
 
   // chunk pipeline for large AllReduces on ordinary buffers
-  static constexpr int kSoloSlots = 8;
   struct Pipeline {
     cudaStream_t s_in = nullptr, s_out = nullptr;
     cudaEvent_t ev_start = nullptr, ev_in[2] = {nullptr, nullptr}, ev_comm[2] = {nullptr, nullptr}, ev_out[2] = {nullptr, nullptr};
-    cudaEvent_t ev_filled[kSoloSlots] = {}, ev_work[kSoloSlots] = {}, ev_done[kSoloSlots] = {};  // one rank only
   };
   std::unique_ptr<Pipeline> pipe_;
-  // single rank with pinned-host buffers: private device staging, a ring of kSoloSlots chunks
-  char* solo_stage_ = nullptr;
-  size_t solo_slot_bytes_ = 0;
+
+  // Single rank with pinned host buffers: a ring of kSoloSlots chunks of device staging, with the side streams and
+  // events that walk it.  Calls that run at once share one ring, each after the one before it, whatever their
+  // streams.  A captured call takes a ring of its own, because its graph replays beside them.
+  static constexpr int kSoloSlots = 8;
+  static constexpr size_t kSoloGraphRings = 4;   // captured calls beyond these rings take the plain kernel
+  struct SoloRing {
+    cudaStream_t s_in = nullptr, s_out = nullptr;
+    cudaEvent_t ev_start = nullptr, ev_last = nullptr;   // ev_last: the end of the last call (not of captured ones)
+    cudaEvent_t ev_filled[kSoloSlots] = {}, ev_work[kSoloSlots] = {}, ev_done[kSoloSlots] = {};
+    char* stage = nullptr;
+    size_t slot_bytes = 0;
+    std::shared_ptr<std::atomic<bool>> in_graph;         // captured rings: a graph holds it
+    unsigned long long capture_id = 0;                   // ... captured into by calls on this stream of this capture
+    cudaStream_t capture_stream = nullptr;
+    void destroy();
+  };
+  SoloRing solo_ring_;
+  std::vector<std::unique_ptr<SoloRing>> solo_graph_rings_;
 
   // plane for ranks that share a GPU: host-synchronised, staging exchanged over CUDA IPC
   bool shared_plane_ = false;

@@ -77,3 +77,96 @@ def test_host_pipeline_in_cuda_graph(comm):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, x * 3.0)
+
+
+def _filled(n, value):
+    return torch.full((n,), float(value)).pin_memory()
+
+
+@pytest.mark.parametrize("scale,mib", [(2.0, 40), (1.0, 160)], ids=["kernel", "copy_engines_only"])
+def test_calls_on_two_streams_do_not_share_the_ring_at_once(comm, scale, mib):
+    """Host buffers large enough that the ring of device slots wraps, on two streams that nothing orders: each call
+    has to wait for the one before it to be through with the slots."""
+    n = (mib << 20) // 4 + 13
+    xs = [_filled(n, 1 + k) for k in range(2)]
+    ys = [[torch.zeros(n).pin_memory() for _ in range(2)] for _ in range(2)]
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    before = comm.stats()["pipelined_calls"]
+    for it in range(2):
+        for k, s in enumerate(streams):
+            comm.all_reduce(xs[k], "sum", out=ys[k][it], scale=scale, stream=s)
+    torch.cuda.synchronize()
+    assert comm.stats()["pipelined_calls"] == before + 4
+    for k in range(2):
+        for it in range(2):
+            assert torch.equal(ys[k][it], xs[k] * scale), (k, it)
+
+
+def test_replay_beside_eager_calls(comm):
+    """A captured pipelined call has a ring of its own: its replays run beside eager calls of the communicator."""
+    n = (40 << 20) // 4 + 5
+    x, y = _filled(n, 3), torch.zeros(n).pin_memory()
+    ex, ey = _filled(n, 5), torch.zeros(n).pin_memory()
+    cap, other = torch.cuda.Stream(), torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    before = comm.stats()["pipelined_calls"]
+    with torch.cuda.stream(cap), torch.cuda.graph(g, stream=cap):
+        comm.all_reduce(x, "sum", out=y, scale=3.0)
+    assert comm.stats()["pipelined_calls"] == before + 1, "the captured call is pipelined, without a warm-up"
+    for _ in range(3):
+        with torch.cuda.stream(cap):
+            g.replay()
+        comm.all_reduce(ex, "sum", out=ey, scale=0.5, stream=other)
+    torch.cuda.synchronize()
+    assert torch.equal(y, x * 3.0) and torch.equal(ey, ex * 0.5)
+
+
+def test_an_eager_call_between_the_calls_of_a_capture(comm):
+    """The side streams of a captured call stay in the capture until it ends; eager calls do not meet them."""
+    n = (20 << 20) // 4
+    x, y, z = _filled(n, 1), torch.zeros(n).pin_memory(), torch.zeros(n).pin_memory()
+    ex, ey = _filled(n, 7), torch.zeros(n).pin_memory()
+    cap, other = torch.cuda.Stream(), torch.cuda.Stream()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(cap), torch.cuda.graph(g, stream=cap, capture_error_mode="relaxed"):
+        comm.all_reduce(x, "sum", out=y, scale=2.0)
+        comm.all_reduce(ex, "sum", out=ey, scale=2.0, stream=other)
+        comm.all_reduce(x, "sum", out=z, scale=4.0)
+    other.synchronize()
+    assert torch.equal(ey, ex * 2.0)
+    assert float(y[0]) == 0.0
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, x * 2.0) and torch.equal(z, x * 4.0)
+
+
+def test_rings_of_graphs_are_bounded_and_reused():
+    import mini_nccl_b200 as mn
+
+    comm = mn.Communicator(1, 0)
+    n = (16 << 20) // 4
+    x = _filled(n, 1)
+    try:
+        def capture(scale):
+            y = torch.zeros(n).pin_memory()
+            g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+            with torch.cuda.stream(s), torch.cuda.graph(g, stream=s):
+                comm.all_reduce(x, "sum", out=y, scale=scale)
+            return g, y
+
+        live = [capture(float(k + 2)) for k in range(5)]
+        assert comm.stats()["pipelined_calls"] == 4, "the fifth live graph holds a plain kernel"
+        for g, _ in live:
+            g.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, x * float(k + 2)) for k, (_, y) in enumerate(live))
+        g = None
+        del live                                             # destroys the graphs: their rings are free again
+        again = [capture(9.0) for _ in range(4)]
+        assert comm.stats()["pipelined_calls"] == 8
+        again[3][0].replay()
+        torch.cuda.synchronize()
+        assert torch.equal(again[3][1], x * 9.0)
+        again = None
+    finally:
+        comm.destroy()
