@@ -19,10 +19,14 @@
 // The reference has no GEMM and no tensor-core code; this exists because the
 // tensor-parallel workload fuses it with the collectives of this library.
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
+#include <memory>
 #include <mutex>
+#include <vector>
 
+#include "core/graph_capture.h"
 #include "kernels/gemm2_kernel.cuh"
 #include "kernels/gemm_small.h"
 #include "mem/cuda_driver.h"
@@ -44,18 +48,38 @@ int pair_mode_from_env() {
 }
 int g_use_pair = pair_mode_from_env();
 uint32_t* g_err_dev[kMaxDevices] = {};  // one error word per device of the process
-// Split-K workspaces: one per (device, stream) that has needed one, so that products on different streams do
-// not add into each other's partial tiles.  At most kSplitPools of them live (20 MB each, for the life of
-// the process); a stream beyond that computes without the split.
+// Split-K workspaces (20 MB each, for the life of the process).  Products that may run at once must not add into
+// each other's partial tiles:
+//   * a product that runs when it is called takes the workspace its stream used last, one of kSplitPools per
+//     device; a stream beyond that many takes over the one that has been idle longest, and waits on the GPU for
+//     the product that used it.  (Streams are told apart by their ids: a handle can be given out again, and
+//     cudaStreamPerThread is another stream in every thread.)
+//   * a captured product may be replayed anywhere, beside anything: it gets one of kSplitGraphPools that its graph
+//     holds until it is destroyed; products of one capture on one stream follow one another and share it.  Where
+//     none is left it is captured without the split.  (Two executable graphs made from one captured graph must not
+//     run at once: they share its workspace as they share the product's output.)
 struct SplitPool {
-  int dev;
-  cudaStream_t stream;
-  float* ws;       // fp32 partial tiles
-  uint32_t* cnt;   // one counter per 32-row quarter
+  float* ws = nullptr;       // fp32 partial tiles
+  uint32_t* cnt = nullptr;   // one counter per 32-row quarter
+  // not captured: the end of the last product, its stream, and when that was
+  cudaEvent_t last = nullptr;
+  unsigned long long stream_id = 0;
+  uint64_t used = 0;
+  // captured: held by a graph, for products on this stream of this capture
+  std::shared_ptr<std::atomic<bool>> in_graph;
+  unsigned long long capture_id = 0;
+  cudaStream_t capture_stream = nullptr;
 };
-constexpr int kSplitPools = 8;
-SplitPool g_split[kSplitPools];
-int g_split_used = 0;
+constexpr size_t kSplitPools = 8, kSplitGraphPools = 8;
+struct SplitPools {
+  std::mutex mu;
+  uint64_t clock = 0;
+  std::vector<SplitPool> live[kMaxDevices], graph[kMaxDevices];
+};
+SplitPools& split_pools() {
+  static auto* pools = new SplitPools;   // outlives the destructors of a process that exits with graphs alive
+  return *pools;
+}
 constexpr int kSplitMaxItems = 80;      // K-slices in flight: at most one per CTA pair
 
 }  // namespace
@@ -99,38 +123,97 @@ uint32_t* error_word() {
   return g_err_dev[dev];
 }
 
-// Workspace of the split last wave: kSplitMaxItems partial tiles of 256 x 256 fp32 (20 MB) and one
-// counter per 32-row quarter.  Allocated the first time a shape is split on `stream` (never under stream
-// capture: call the GEMM once on that stream before capturing).  False: no split then.
-bool split_workspace(cudaStream_t stream, float** ws, uint32_t** cnt) {
-  std::lock_guard<std::mutex> lk(g_mu);
-  const int dev = current_device_slot();
-  for (int i = 0; i < g_split_used; ++i) {
-    if (g_split[i].dev == dev && g_split[i].stream == stream) {
-      *ws = g_split[i].ws;
-      *cnt = g_split[i].cnt;
+namespace {
+
+// kSplitMaxItems partial tiles of 256 x 256 fp32 and one zeroed counter per 32-row quarter.
+bool create_split_pool(SplitPool* p, bool captured) {
+  AllowAllocationsWhileCapturing allow;
+  constexpr size_t kCntBytes = size_t(kSplitMaxItems) * 8 * 4;
+  cudaStream_t s = nullptr;   // the zeroes must not be captured, nor wait behind other work
+  bool ok = cudaMalloc(&p->ws, size_t(kSplitMaxItems) * 256 * 256 * 4) == cudaSuccess && cudaMalloc(&p->cnt, kCntBytes) == cudaSuccess &&
+            cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess && cudaMemsetAsync(p->cnt, 0, kCntBytes, s) == cudaSuccess &&
+            cudaStreamSynchronize(s) == cudaSuccess;
+  if (ok && !captured) ok = cudaEventCreateWithFlags(&p->last, cudaEventDisableTiming) == cudaSuccess;
+  if (s) cudaStreamDestroy(s);
+  if (ok) return true;
+  (void)cudaGetLastError();
+  if (p->ws) cudaFree(p->ws);
+  if (p->cnt) cudaFree(p->cnt);
+  *p = SplitPool{};
+  return false;
+}
+
+// A workspace for one product on `stream`, taken before its launch; launched() goes after it.  Other threads wait
+// in between, so that none takes the workspace over before the product is in its stream.
+class SplitLease {
+ public:
+  bool take(cudaStream_t stream) {
+    SplitPools& all = split_pools();
+    lock_ = std::unique_lock<std::mutex>(all.mu);
+    const int dev = current_device_slot();
+    const CaptureInfo cap = capture_info(stream);
+    return cap.active ? take_captured(all.graph[dev], cap, stream) : take_live(all.live[dev], stream);
+  }
+  float* ws() const { return pool_->ws; }
+  uint32_t* cnt() const { return pool_->cnt; }
+  void launched(cudaStream_t stream) {
+    if (pool_ == nullptr || pool_->last == nullptr) return;
+    if (cudaEventRecord(pool_->last, stream) != cudaSuccess) (void)cudaGetLastError();
+    pool_->stream_id = id_;
+    pool_->used = ++split_pools().clock;
+  }
+
+ private:
+  bool take_live(std::vector<SplitPool>& pools, cudaStream_t stream) {
+    if (cudaStreamGetId(stream, &id_) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    SplitPool* oldest = nullptr;
+    for (SplitPool& p : pools) {
+      if (p.used != 0 && p.stream_id == id_) return (pool_ = &p) != nullptr;
+      if (oldest == nullptr || p.used < oldest->used) oldest = &p;
+    }
+    SplitPool fresh;
+    if (pools.size() < kSplitPools && create_split_pool(&fresh, false)) {
+      pools.push_back(fresh);
+      pool_ = &pools.back();
       return true;
     }
+    if (oldest == nullptr) return false;
+    if (cudaStreamWaitEvent(stream, oldest->last, 0) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    pool_ = oldest;
+    return true;
   }
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (g_split_used == kSplitPools || cudaStreamIsCapturing(stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) {
-    (void)cudaGetLastError();
-    return false;
+  bool take_captured(std::vector<SplitPool>& pools, const CaptureInfo& cap, cudaStream_t stream) {
+    SplitPool* idle = nullptr;
+    for (SplitPool& p : pools) {
+      if (!p.in_graph->load(std::memory_order_acquire)) idle = &p;
+      else if (p.capture_id == cap.id && p.capture_stream == stream) return (pool_ = &p) != nullptr;
+    }
+    if (idle == nullptr) {
+      SplitPool fresh;
+      if (pools.size() >= kSplitGraphPools || !create_split_pool(&fresh, true)) return false;
+      fresh.in_graph = std::make_shared<std::atomic<bool>>(false);
+      pools.push_back(fresh);
+      idle = &pools.back();
+    }
+    if (!hold_while_graph_lives(cap.graph, idle->in_graph)) return false;
+    idle->capture_id = cap.id;
+    idle->capture_stream = stream;
+    pool_ = idle;
+    return true;
   }
-  SplitPool p{dev, stream, nullptr, nullptr};
-  if (cudaMalloc(&p.ws, size_t(kSplitMaxItems) * 256 * 256 * 4) != cudaSuccess ||
-      cudaMalloc(&p.cnt, size_t(kSplitMaxItems) * 8 * 4) != cudaSuccess ||
-      cudaMemset(p.cnt, 0, size_t(kSplitMaxItems) * 8 * 4) != cudaSuccess || cudaStreamSynchronize(nullptr) != cudaSuccess) {
-    (void)cudaGetLastError();
-    if (p.ws) cudaFree(p.ws);
-    if (p.cnt) cudaFree(p.cnt);
-    return false;
-  }
-  g_split[g_split_used++] = p;
-  *ws = p.ws;
-  *cnt = p.cnt;
-  return true;
-}
+
+  std::unique_lock<std::mutex> lock_;
+  SplitPool* pool_ = nullptr;
+  unsigned long long id_ = 0;
+};
+
+}  // namespace
 
 // Split-K plan of the CTA-pair kernel: tiles2 tiles on n_pairs pairs, num_kb k-blocks per tile.  When
 // the last wave holds at most half as many tiles as there are pairs, each of its tiles is cut into at
@@ -315,12 +398,15 @@ int run_gemm(const char* who, const void* A, const void* B, void* C, int M, int 
   g.wait_budget_ns = 2000000000ull;
   g.group_m = 8;
   int grid;
+  SplitLease lease;
   if (pair) {
     const int tiles2 = ((M + 2 * kBM - 1) / (2 * kBM)) * ((N + kBN - 1) / kBN);
     grid = std::min(2 * tiles2, sms & ~1);
     const int pairs = std::min(grid / 2, out == kOutSwiGlu ? max_pairs<SwiGluEpilogue>() : max_pairs<StoreEpilogue<false>>());
     int first = 0, slices = 0, per = 0;
-    if (plan_split(tiles2, pairs, (K + kBK - 1) / kBK, &first, &slices, &per) && split_workspace(stream, &g.split_ws, &g.split_cnt)) {
+    if (plan_split(tiles2, pairs, (K + kBK - 1) / kBK, &first, &slices, &per) && lease.take(stream)) {
+      g.split_ws = lease.ws();
+      g.split_cnt = lease.cnt();
       g.split_first = first;
       g.split_s = slices;
       g.split_kb = per;
@@ -333,6 +419,7 @@ int run_gemm(const char* who, const void* A, const void* B, void* C, int M, int 
   if (out == kOutF32) e = fire(StoreEpilogue<true>{});
   else if (out == kOutSwiGlu) e = fire(SwiGluEpilogue{bn / 32});
   else e = fire(StoreEpilogue<false>{});
+  if (e == cudaSuccess) lease.launched(stream);
   return e == cudaSuccess ? 0 : static_cast<int>(e) + 1000;
 }
 
