@@ -192,15 +192,21 @@ _EXT = None
 
 def ext():
     """The PyTorch extension behind the frequent calls (csrc/torch/ext.cpp), bound to the library that
-    :func:`lib` has loaded.  Built on first use if its file is missing."""
+    :func:`lib` has loaded.  Built on first use if its file is missing; with a PyTorch it cannot be built
+    against (one without CUDA) the same calls through ctypes."""
     global _EXT
     if _EXT is not None:
         return _EXT
     import torch  # noqa: F401  (its shared libraries must be in the process first)
 
     L = lib()
+    from . import build as _build
+    if _build.torch_dir() is None:
+        from ._ctypes_calls import Calls
+
+        _EXT = Calls(L)
+        return _EXT
     if not (_HERE / "_torch_ext.so").exists():
-        from . import build as _build
         _build.build_torch_ext()
     from . import _torch_ext
 

@@ -113,24 +113,33 @@ def lib_path() -> Path:
     return LIBDIR / "libmini_nccl.so"
 
 
-def build_torch_ext(verbose: bool = False) -> Path | None:
-    """The CPython extension behind the binding's frequent calls (csrc/torch/ext.cpp), compiled against the
-    installed PyTorch; None where there is none (the ctypes binding itself does not need it)."""
+def torch_dir() -> Path | None:
+    """Where the PyTorch is that the extension can be built against: one with CUDA."""
     import importlib.util
-    import sysconfig
 
     spec = importlib.util.find_spec("torch")
     if spec is None or not spec.submodule_search_locations:
         return None
-    torch_dir = Path(spec.submodule_search_locations[0])
+    d = Path(spec.submodule_search_locations[0])
+    return d if (d / "lib" / "libc10_cuda.so").exists() else None
+
+
+def build_torch_ext(verbose: bool = False) -> Path | None:
+    """The CPython extension behind the binding's frequent calls (csrc/torch/ext.cpp), compiled against the
+    installed PyTorch; None where there is none with CUDA (the same calls then go through ctypes)."""
+    import sysconfig
+
+    torch_at = torch_dir()
+    if torch_at is None:
+        return None
     out = ROOT / "mini_nccl_b200" / "_torch_ext.so"
     src = CSRC / "torch" / "ext.cpp"
     newest = max(src.stat().st_mtime, *(h.stat().st_mtime for h in (ROOT / "include").glob("*.h")))
     if out.exists() and out.stat().st_mtime >= newest:
         return out
     cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", "-shared", *_common_includes(),
-           "-isystem", str(torch_dir / "include"), "-isystem", str(torch_dir / "include" / "torch" / "csrc" / "api" / "include"),
-           "-I", sysconfig.get_paths()["include"], str(src), "-o", str(out), "-L", str(torch_dir / "lib"),
+           "-isystem", str(torch_at / "include"), "-isystem", str(torch_at / "include" / "torch" / "csrc" / "api" / "include"),
+           "-I", sysconfig.get_paths()["include"], str(src), "-o", str(out), "-L", str(torch_at / "lib"),
            "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
     if verbose:
         print(" ".join(cmd), flush=True)
