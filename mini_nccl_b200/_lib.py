@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import warnings
 from pathlib import Path
 
 _HERE = Path(__file__).resolve().parent
@@ -193,7 +194,7 @@ _EXT = None
 def ext():
     """The PyTorch extension behind the frequent calls (csrc/torch/ext.cpp), bound to the library that
     :func:`lib` has loaded.  Built on first use if its file is missing; with a PyTorch it cannot be built
-    against (one without CUDA) the same calls through ctypes."""
+    against (one without CUDA), or where MINI_NCCL_NO_BUILD=1 forbids it, the same calls through ctypes."""
     global _EXT
     if _EXT is not None:
         return _EXT
@@ -201,12 +202,16 @@ def ext():
 
     L = lib()
     from . import build as _build
-    if _build.torch_dir() is None:
+    no_build = os.environ.get("MINI_NCCL_NO_BUILD") == "1"
+    missing = not (_HERE / "_torch_ext.so").exists()
+    if _build.torch_dir() is None or (missing and no_build):
         from ._ctypes_calls import Calls
 
+        if missing and no_build:
+            warnings.warn("the PyTorch extension is missing and MINI_NCCL_NO_BUILD=1: its calls go through ctypes")
         _EXT = Calls(L)
         return _EXT
-    if not (_HERE / "_torch_ext.so").exists():
+    if missing:
         _build.build_torch_ext()
     from . import _torch_ext
 

@@ -56,6 +56,23 @@ comm.destroy()
     assert [p.returncode for p in procs] == [0, 0], outs
 
 
+def test_no_build_is_honoured():
+    """MINI_NCCL_NO_BUILD=1: a missing extension is not compiled; its calls go through ctypes, and a warning says so."""
+    _run("""
+import warnings
+import mini_nccl_b200.build as b
+from mini_nccl_b200 import _lib
+def never(*a, **k): raise AssertionError("built although MINI_NCCL_NO_BUILD=1")
+b.build_torch_ext = never
+_lib.lib()
+_lib._HERE = _lib._HERE / "nowhere"        # the extension's file is missing
+with warnings.catch_warnings(record=True) as w:
+    warnings.simplefilter("always")
+    assert type(_lib.ext()).__name__ == "Calls"
+assert any("MINI_NCCL_NO_BUILD" in str(x.message) for x in w)
+""", {"MINI_NCCL_NO_BUILD": "1"})
+
+
 @pytest.mark.gpu
 def test_ctypes_calls_give_what_the_extension_gives():
     import mini_nccl_b200 as mn
