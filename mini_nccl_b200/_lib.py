@@ -8,6 +8,7 @@ symbol names with its own signature, reference: include/mini_nccl_api.h:57).
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 import warnings
 from pathlib import Path
@@ -202,18 +203,21 @@ def ext():
 
     L = lib()
     from . import build as _build
-    no_build = os.environ.get("MINI_NCCL_NO_BUILD") == "1"
-    missing = not (_HERE / "_torch_ext.so").exists()
-    if _build.torch_dir() is None or (missing and no_build):
+    path = _build.torch_ext_path()
+    if path is not None and not path.exists():
+        if os.environ.get("MINI_NCCL_NO_BUILD") == "1":
+            warnings.warn("the PyTorch extension is missing and MINI_NCCL_NO_BUILD=1: its calls go through ctypes")
+            path = None
+        else:
+            _build.build_torch_ext()
+    if path is None:
         from ._ctypes_calls import Calls
 
-        if missing and no_build:
-            warnings.warn("the PyTorch extension is missing and MINI_NCCL_NO_BUILD=1: its calls go through ctypes")
         _EXT = Calls(L)
         return _EXT
-    if missing:
-        _build.build_torch_ext()
-    from . import _torch_ext
+    spec = importlib.util.spec_from_file_location(f"{__package__}._torch_ext", path)
+    _torch_ext = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(_torch_ext)
 
     address = lambda name: C.cast(getattr(L, name), C.c_void_p).value if hasattr(L, name) else 0
     _torch_ext.bind(address("mncclAllReduceEx"), address("mncclCommGetAsyncError"), address("mncclGemmBf16"),

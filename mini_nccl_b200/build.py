@@ -28,6 +28,7 @@ CSRC = ROOT / "csrc"
 BUILD = ROOT / "build"
 LIBDIR = ROOT / "mini_nccl_b200" / "lib"
 BINDIR = ROOT / "mini_nccl_b200" / "bin"
+EXTDIR = ROOT / "mini_nccl_b200"
 
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
@@ -124,22 +125,38 @@ def torch_dir() -> Path | None:
     return d if (d / "lib" / "libc10_cuda.so").exists() else None
 
 
+def torch_ext_path() -> Path | None:
+    """The extension's file for the installed PyTorch and this Python, or None where there is none with CUDA.  Its
+    name holds both versions and a hash of the source: a file made for another PyTorch, another Python or from
+    another source is never taken for it."""
+    import re
+    import sysconfig
+
+    at = torch_dir()
+    if at is None:
+        return None
+    version = re.search(r"^__version__ = '([^']+)'", (at / "version.py").read_text(), re.M).group(1)
+    tag = f"{version}-{sysconfig.get_config_var('SOABI')}"
+    sources = [CSRC / "torch" / "ext.cpp", *sorted((ROOT / "include").glob("*.h"))]
+    if not sources[0].exists():    # a tree without sources: what was built for these versions
+        built = sorted(EXTDIR.glob(f"_torch_ext-{tag}-*.so"))
+        return built[-1] if built else None
+    digest = hashlib.sha1(b"".join(p.read_bytes() for p in sources)).hexdigest()[:8]
+    return EXTDIR / f"_torch_ext-{tag}-{digest}.so"
+
+
 def build_torch_ext(verbose: bool = False) -> Path | None:
     """The CPython extension behind the binding's frequent calls (csrc/torch/ext.cpp), compiled against the
     installed PyTorch; None where there is none with CUDA (the same calls then go through ctypes)."""
     import sysconfig
 
-    torch_at = torch_dir()
-    if torch_at is None:
-        return None
-    out = ROOT / "mini_nccl_b200" / "_torch_ext.so"
-    src = CSRC / "torch" / "ext.cpp"
-    newest = max(src.stat().st_mtime, *(h.stat().st_mtime for h in (ROOT / "include").glob("*.h")))
-    if out.exists() and out.stat().st_mtime >= newest:
+    out = torch_ext_path()
+    if out is None or out.exists():
         return out
+    torch_at = torch_dir()
     cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", "-shared", *_common_includes(),
            "-isystem", str(torch_at / "include"), "-isystem", str(torch_at / "include" / "torch" / "csrc" / "api" / "include"),
-           "-I", sysconfig.get_paths()["include"], str(src), "-o", str(out), "-L", str(torch_at / "lib"),
+           "-I", sysconfig.get_paths()["include"], str(CSRC / "torch" / "ext.cpp"), "-o", str(out), "-L", str(torch_at / "lib"),
            "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
     if verbose:
         print(" ".join(cmd), flush=True)

@@ -65,12 +65,38 @@ from mini_nccl_b200 import _lib
 def never(*a, **k): raise AssertionError("built although MINI_NCCL_NO_BUILD=1")
 b.build_torch_ext = never
 _lib.lib()
-_lib._HERE = _lib._HERE / "nowhere"        # the extension's file is missing
+b.EXTDIR = b.EXTDIR / "nowhere"             # the extension's file is missing
 with warnings.catch_warnings(record=True) as w:
     warnings.simplefilter("always")
     assert type(_lib.ext()).__name__ == "Calls"
 assert any("MINI_NCCL_NO_BUILD" in str(x.message) for x in w)
 """, {"MINI_NCCL_NO_BUILD": "1"})
+
+
+def test_the_file_is_that_of_this_pytorch_python_and_source(tmp_path):
+    _run("""
+import sys, sysconfig, torch
+from pathlib import Path
+import mini_nccl_b200.build as b
+from mini_nccl_b200 import _lib
+path = b.torch_ext_path()
+assert torch.__version__ in path.name and sysconfig.get_config_var("SOABI") in path.name
+assert Path(_lib.ext().__file__) == path, "the file loaded is the one of this name"
+tmp = Path(sys.argv[1]) if len(sys.argv) > 1 else Path(%r)
+other = tmp / "torch"
+(other / "lib").mkdir(parents=True)
+(other / "lib" / "libc10_cuda.so").touch()
+(other / "version.py").write_text("__version__ = '9.9.9'\\n")
+real = b.torch_dir
+b.torch_dir = lambda: other
+assert "9.9.9" in b.torch_ext_path().name and b.torch_ext_path() != path, "another PyTorch, another file"
+b.torch_dir = real
+src = b.CSRC
+b.CSRC = tmp / "csrc"
+(b.CSRC / "torch").mkdir(parents=True)
+(b.CSRC / "torch" / "ext.cpp").write_text((src / "torch" / "ext.cpp").read_text() + "// edited")
+assert b.torch_ext_path() != path, "an edited source, another file"
+""" % str(tmp_path))
 
 
 @pytest.mark.gpu
