@@ -16,6 +16,7 @@ for C / C++ users.
 from __future__ import annotations
 
 import concurrent.futures as cf
+import fcntl
 import hashlib
 import os
 import shutil
@@ -154,15 +155,27 @@ def build_torch_ext(verbose: bool = False) -> Path | None:
     if out is None or out.exists():
         return out
     torch_at = torch_dir()
-    cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", "-shared", *_common_includes(),
-           "-isystem", str(torch_at / "include"), "-isystem", str(torch_at / "include" / "torch" / "csrc" / "api" / "include"),
-           "-I", sysconfig.get_paths()["include"], str(CSRC / "torch" / "ext.cpp"), "-o", str(out), "-L", str(torch_at / "lib"),
-           "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
-    if verbose:
-        print(" ".join(cmd), flush=True)
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"build of the PyTorch extension failed\n{r.stderr}")
+    BUILD.mkdir(exist_ok=True)
+    # Ranks that start together and find the file missing: one compiles, the others wait for it, and nobody sees a
+    # half-written file under the final name.
+    with open(BUILD / "torch_ext.lock", "w") as lock:
+        fcntl.flock(lock, fcntl.LOCK_EX)
+        if out.exists():
+            return out
+        part = out.with_suffix(f".{os.getpid()}.part")
+        cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", "-shared", *_common_includes(),
+               "-isystem", str(torch_at / "include"), "-isystem", str(torch_at / "include" / "torch" / "csrc" / "api" / "include"),
+               "-I", sysconfig.get_paths()["include"], str(CSRC / "torch" / "ext.cpp"), "-o", str(part), "-L", str(torch_at / "lib"),
+               "-ltorch_python", "-ltorch_cpu", "-lc10_cuda", "-lc10"]
+        if verbose:
+            print(" ".join(cmd), flush=True)
+        try:
+            r = subprocess.run(cmd, capture_output=True, text=True)
+            if r.returncode != 0:
+                raise RuntimeError(f"build of the PyTorch extension failed\n{r.stderr}")
+            os.replace(part, out)
+        finally:
+            part.unlink(missing_ok=True)
     return out
 
 

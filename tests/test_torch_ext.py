@@ -99,6 +99,39 @@ assert b.torch_ext_path() != path, "an edited source, another file"
 """ % str(tmp_path))
 
 
+def test_processes_that_start_together_build_it_once_and_never_see_half_a_file(tmp_path):
+    """A stand-in compiler that writes its output in two halves, a moment apart; three processes find the file
+    missing at the same time."""
+    fake = tmp_path / "bin" / "g++"
+    fake.parent.mkdir()
+    fake.write_text('#!/bin/sh\necho run >> "%s/runs"\nwhile [ "$1" != "-o" ]; do shift; done\nprintf first > "$2"\nsleep 1\n'
+                    'printf second >> "$2"\n' % tmp_path)
+    fake.chmod(0o755)
+    code = """
+import sys, threading
+from pathlib import Path
+import mini_nccl_b200.build as b
+b.EXTDIR = b.BUILD = Path(%r)
+path, seen, done = b.torch_ext_path(), [], threading.Event()
+def watch():
+    while not done.is_set():
+        if path.exists(): seen.append(path.read_text())
+t = threading.Thread(target=watch); t.start()
+assert b.build_torch_ext() == path
+done.set(); t.join()
+assert path.read_text() == "firstsecond" and set(seen) <= {"firstsecond"}, set(seen)
+""" % str(tmp_path)
+    import os
+
+    env = dict(os.environ, PYTHONPATH=str(ROOT), PATH=f"{fake.parent}:{os.environ['PATH']}")
+    procs = [subprocess.Popen([sys.executable, "-c", code], env=env, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+             for _ in range(3)]
+    outs = [p.communicate(timeout=120)[0] for p in procs]
+    assert [p.returncode for p in procs] == [0, 0, 0], outs
+    assert (tmp_path / "runs").read_text() == "run\n"
+    assert sorted(p.suffix for p in tmp_path.glob("_torch_ext*")) == [".so"]
+
+
 @pytest.mark.gpu
 def test_ctypes_calls_give_what_the_extension_gives():
     import mini_nccl_b200 as mn
