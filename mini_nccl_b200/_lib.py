@@ -195,7 +195,7 @@ _EXT = None
 def ext():
     """The PyTorch extension behind the frequent calls (csrc/torch/ext.cpp), bound to the library that
     :func:`lib` has loaded.  Built on first use if its file is missing; with a PyTorch it cannot be built
-    against (one without CUDA), or where MINI_NCCL_NO_BUILD=1 forbids it, the same calls through ctypes."""
+    against (one without CUDA), or where that fails or MINI_NCCL_NO_BUILD=1 forbids it, the same calls through ctypes."""
     global _EXT
     if _EXT is not None:
         return _EXT
@@ -205,11 +205,15 @@ def ext():
     from . import build as _build
     path = _build.torch_ext_path()
     if path is not None and not path.exists():
-        if os.environ.get("MINI_NCCL_NO_BUILD") == "1":
-            warnings.warn("the PyTorch extension is missing and MINI_NCCL_NO_BUILD=1: its calls go through ctypes")
+        why = "MINI_NCCL_NO_BUILD=1" if os.environ.get("MINI_NCCL_NO_BUILD") == "1" else None
+        if why is None:
+            try:
+                _build.build_torch_ext()
+            except (RuntimeError, OSError) as e:   # no compiler, or one that fails
+                why = str(e)
+        if why is not None:
+            warnings.warn(f"the PyTorch extension is missing ({why}): its calls go through ctypes")
             path = None
-        else:
-            _build.build_torch_ext()
     if path is None:
         from ._ctypes_calls import Calls
 

@@ -73,6 +73,22 @@ assert any("MINI_NCCL_NO_BUILD" in str(x.message) for x in w)
 """, {"MINI_NCCL_NO_BUILD": "1"})
 
 
+def test_without_a_compiler_the_calls_go_through_ctypes(tmp_path):
+    _run("""
+import os, warnings, torch
+from pathlib import Path
+import mini_nccl_b200.build as b
+from mini_nccl_b200 import _lib
+b.EXTDIR = b.BUILD = Path(%r)
+_lib.lib()
+os.environ["PATH"] = ""                     # no g++
+with warnings.catch_warnings(record=True) as w:
+    warnings.simplefilter("always")
+    assert type(_lib.ext()).__name__ == "Calls"
+assert any("g++" in str(x.message) for x in w)
+""" % str(tmp_path))
+
+
 def test_the_file_is_that_of_this_pytorch_python_and_source(tmp_path):
     _run("""
 import sys, sysconfig, torch
