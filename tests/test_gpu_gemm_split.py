@@ -76,6 +76,28 @@ def test_products_on_the_per_thread_default_streams(product):
     _check(outs, want)
 
 
+def test_the_first_cuda_call_of_a_thread(product):
+    """A thread that has made no CUDA call has no context yet; the product is its first."""
+    from mini_nccl_b200.ops import gemm_bf16
+
+    a, b, want, _ = product
+    out = torch.zeros_like(want)
+    torch.cuda.synchronize()
+    failed = []
+
+    def work():
+        try:
+            gemm_bf16(a, b, out=out, stream=0)
+        except RuntimeError as e:
+            failed.append(e)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    assert not failed, failed
+    _check([out], want)
+
+
 def _capture(a, b, out, stream):
     from mini_nccl_b200.ops import gemm_bf16
 
