@@ -254,7 +254,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tile_coords(g, t, tiles_m, tiles_n, &tm, &tn);
       const uint32_t buf = local & 1u;
       const uint32_t acc_ph = (local >> 1) & 1u;
-      if (!mbar_wait(smem_u32(&ctl->tmem_full[buf]), acc_ph, &ctl->abort, budget)) { ok = false; break; }
+      if (!mbar_wait_warp(smem_u32(&ctl->tmem_full[buf]), acc_ph, &ctl->abort, budget)) { ok = false; break; }
       tc_fence_after_sync();
       const int row = tm * kBM + q * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * kBN;

@@ -176,7 +176,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
   const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16);
   bool ok = true;
   if (warp >= 2) {
-    ok = mbar_wait(smem_u32(&ctl->done), 0, &ctl->abort, g.wait_budget_ns);
+    ok = mbar_wait_warp(smem_u32(&ctl->done), 0, &ctl->abort, g.wait_budget_ns);
     tc_fence_after_sync();
   }
   constexpr int kPiece = TN < 32 ? TN : 32;  // accumulator columns per TMEM load
