@@ -188,7 +188,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       const int tm = tm2 * 2 + static_cast<int>(cta);
       const uint32_t buf = local & 1u;
       const uint32_t acc_ph = (local >> 1) & 1u;
-      if (!mbar_wait_warp(smem_u32(&ctl->tmem_full[buf]), acc_ph, &ctl->abort, budget)) { ok = false; break; }
+      if (!accumulator_wait<Epilogue>(smem_u32(&ctl->tmem_full[buf]), acc_ph, &ctl->abort, budget)) { ok = false; break; }
       tc_fence_after_sync();
       const int row = tm * kBM + q * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * kBN;

@@ -50,11 +50,6 @@ __device__ __forceinline__ void st_release_sys_u32(uint32_t* p, uint32_t v) {
 __device__ __forceinline__ void red_release_sys_add(uint32_t* p, uint32_t v) {
   asm volatile("red.release.sys.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
-__device__ __forceinline__ void epilogue_warps_sync() {
-  // the four epilogue warps (128 threads) on named barrier 1
-  asm volatile("bar.sync 1, 128;" ::: "memory");
-}
-
 // Bounded wait for *p >= target (wrap-safe) with system-scope acquire.  Gives up when the budget runs
 // out, when another role of the CTA has given up (*abort_flag) or when the communicator's abort word
 // is set (the watchdog of this or of another local rank tripped): the kernel then winds down and the
@@ -82,6 +77,7 @@ __device__ __forceinline__ bool wait_flag_sys(const uint32_t* p, uint32_t target
 // ------------------------------------------------------------------ GEMM -> reduce-scatter
 
 struct RsEpilogue {
+  static constexpr bool kWarpsMeet = true;
   static constexpr int kWarpSmemBytes = kEpiWarpBytes;
   static constexpr int kSingleStages = kStages;
   static constexpr int kPairStages = 6;
@@ -212,8 +208,8 @@ struct RsEpilogue {
         if (tid < nranks) {
           wait_flag_sys(flags[rank] + (static_cast<size_t>(tid) * tiles_m_local + ltm) * tiles_n + tn, epoch, abort_flag, g);
         }
-        epilogue_warps_sync();
-        if (*abort_flag != 0u) return;
+        // (a flag read after the barrier could be set in between: some threads would leave, the others wait)
+        if (epilogue_warps_any(*abort_flag != 0u)) return;
         last_tile = tile;
       }
       const int row0 = ltm * kBM + part * kRows;
@@ -330,6 +326,7 @@ struct RsEpilogue {
 // ------------------------------------------------------------------ all-gather -> GEMM
 
 struct AgEpilogue {
+  static constexpr bool kWarpsMeet = false;
   int rank, nranks;
   int rows_per_rank;                 // M / nranks, a multiple of 128
   int lda;                           // row stride of the gather buffers, elements

@@ -99,6 +99,28 @@ __device__ __forceinline__ bool rows_ready(const GemmArgs& g, uint32_t epoch, in
   return __all_sync(0xffffffffu, ok) != 0;
 }
 
+// The four epilogue warps (128 threads) on named barrier 1: a plain meeting, and one that also tells all of them
+// whether `x` holds for any.
+__device__ __forceinline__ void epilogue_warps_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+__device__ __forceinline__ bool epilogue_warps_any(bool x) {
+  uint32_t any;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.or.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(any)
+      : "r"(x ? 1u : 0u)
+      : "memory");
+  return any != 0u;
+}
+
+// An epilogue warp's wait for a finished accumulator.  Where the epilogue's warps meet at barriers after a tile, all
+// four go by one answer: a warp that gave up alone would leave the others at a barrier for good.
+template <typename Epilogue>
+__device__ __forceinline__ bool accumulator_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint64_t budget_ns) {
+  const bool ok = mbar_wait_warp(bar, parity, abort_flag, budget_ns);
+  if constexpr (Epilogue::kWarpsMeet) return !epilogue_warps_any(!ok);
+  return ok;
+}
+
 struct __align__(8) SharedCtl {
   uint64_t full[kStages];
   uint64_t empty[kStages];
@@ -254,7 +276,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       tile_coords(g, t, tiles_m, tiles_n, &tm, &tn);
       const uint32_t buf = local & 1u;
       const uint32_t acc_ph = (local >> 1) & 1u;
-      if (!mbar_wait_warp(smem_u32(&ctl->tmem_full[buf]), acc_ph, &ctl->abort, budget)) { ok = false; break; }
+      if (!accumulator_wait<Epilogue>(smem_u32(&ctl->tmem_full[buf]), acc_ph, &ctl->abort, budget)) { ok = false; break; }
       tc_fence_after_sync();
       const int row = tm * kBM + q * 32 + lane;
       const uint32_t taddr = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * kBN;

@@ -110,6 +110,7 @@ __host__ __device__ __forceinline__ void tile_coords(const GemmArgs& g, int t, i
 // Plain epilogue: convert and store the accumulator tile to C.
 template <bool OUT_F32>
 struct StoreEpilogue {
+  static constexpr bool kWarpsMeet = false;  // whether tile_done / after_tiles have barriers of the four warps
   // what the kernels size their shared memory by: scratch per epilogue warp, TMA ring depth of the
   // single-CTA and of the CTA-pair kernel
   static constexpr int kWarpSmemBytes = kEpiWarpBytes;
@@ -221,6 +222,7 @@ struct StoreEpilogue {
 // C is [M, N / 2]: the (gate | up) matrix never reaches memory, the kernel writes half the bytes and the
 // separate elementwise pass disappears.  N is a multiple of 32, C and its rows are 16-byte aligned.
 struct SwiGluEpilogue {
+  static constexpr bool kWarpsMeet = false;  // whether tile_done / after_tiles have barriers of the four warps
   static constexpr int kWarpSmemBytes = kEpiWarpBytes;
   static constexpr int kSingleStages = kStages;
   static constexpr int kPairStages = 6;

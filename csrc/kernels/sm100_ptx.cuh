@@ -84,10 +84,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 
 // The same for a whole warp: one answer for all lanes.  When the budget runs out single lanes may still see the
 // phase complete, so whatever a warp does together after a wait (tcgen05.ld, cluster barriers, shuffles) needs this
-// form.  Roles that issue TMA loads or MMAs walk their loops
-// as whole warps and let one elected lane issue, because stage addresses and descriptors then stay in
-// uniform registers; inside `if (lane == 0)` every MMA and every load first moves its operands over
-// (measured: 0.27 us per k-block of four small MMAs and two loads, against 0.16).
+// form.  Roles that issue TMA loads or MMAs walk their loops as whole warps and let one elected lane issue, because
+// stage addresses and descriptors then stay in uniform registers; inside `if (lane == 0)` every MMA and every load
+// first moves its operands over (measured: 0.27 us per k-block of four small MMAs and two loads, against 0.16).
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
                                                uint64_t budget_ns) {
   return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, budget_ns)) != 0;
