@@ -123,7 +123,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    uint32_t s = 0, ph = 1;
+    uint32_t it = 0, s = 0, ph = 1;  // ring position over all k-blocks: count, stage, parity to wait for
     bool ok = true;
     const uint32_t leader_full = map_to_cta(smem_u32(&ctl->full[0]), 0);
     for (int t = pair; t < num_items && ok; t += n_pairs) {
@@ -132,7 +132,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       tile_coords(g2, w.tile, tiles_m2, tiles_n, &tm2, &tn);
       const int tm = tm2 * 2 + static_cast<int>(cta);
       if (g.a_ready != nullptr && !rows_ready(g, epoch, tm, leader, &ctl->abort)) { ok = false; break; }
-      for (int kb = w.kb0; kb < w.kb1; ++kb) {
+      for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
         if (!mbar_wait_warp(smem_u32(&ctl->empty[0]) + s * 8u, ph, &ctl->abort, budget)) { ok = false; break; }
         if (leader) {
           const uint32_t full = leader_full + s * 8u;
@@ -143,6 +143,12 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         }
         if (++s == NS) { s = 0; ph ^= 1u; }
       }
+    }
+    // Both CTAs' loads count on the leader's barriers, and its partner stays until the cluster barrier at the end.  Where
+    // this producer gave up, the partner may be up to a ring ahead.
+    if (cta == 0) {
+      loads_land(&ctl->full[0], NS, it, budget);
+      if (!ok) loads_land(&ctl->full[0], NS, it + NS, budget);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (leader CTA only)

@@ -426,7 +426,10 @@ struct AgEpilogue {
         }
       }
       bulk_wait_all();            // the rows of this quarter are written
-      if (!ok) return;
+      if (!ok) {
+        loads_land(s_full, static_cast<uint32_t>(slots), n_loaded, g.wait_budget_ns);
+        return;
+      }
       fence_proxy_async_all();    // writes of the async proxy before the release below
       red_release_sys_add(ready[peer] + (row0 / kBM), 1u);
     }

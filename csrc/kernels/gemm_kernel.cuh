@@ -121,6 +121,14 @@ __device__ __forceinline__ bool accumulator_wait(uint32_t bar, uint32_t parity, 
   return ok;
 }
 
+// Last step of a producer that has issued `n` loads into a ring of `stages`: the ones still in flight land (bounded),
+// whoever gave up first, before this CTA's shared memory goes away.  After a run without failures they have landed.
+__device__ __forceinline__ void loads_land(uint64_t* full, uint32_t stages, uint32_t n, uint64_t budget_ns) {
+  volatile uint32_t late = 0;   // its own: the CTA's abort flag may be set, which would end every wait at once
+  for (uint32_t j = n > stages ? n - stages : 0; j < n; ++j)
+    mbar_wait(smem_u32(full + j % stages), (j / stages) & 1u, &late, budget_ns);
+}
+
 struct __align__(8) SharedCtl {
   uint64_t full[kStages];
   uint64_t empty[kStages];
@@ -226,15 +234,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         if (++s == NS) { s = 0; ph ^= 1u; }
       }
     }
-    // Wind-down after a failed wait: let copies that are still in flight land
-    // before the CTA (and its shared memory) goes away.
-    if (!ok) {
-      for (uint32_t back = 0; back < NS && back < it; ++back) {
-        const uint32_t j = it - 1 - back;
-        mbar_wait(smem_u32(&ctl->full[j % NS]), (j / NS) & 1u, &ctl->abort /*already set*/, 0);
-        // (budget 0: one more try each; the data either landed or the MMA side consumed it)
-      }
-    }
+    loads_land(&ctl->full[0], NS, it, budget);
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
     constexpr uint32_t idesc = make_idesc_bf16(kBM, BN);

@@ -139,11 +139,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
       if (leader) load(i, s);
       if (++s == NS) { s = 0; ph ^= 1u; }
     }
-    // A wait gave up: what is still in flight lands (bounded) before this shared memory goes away.
-    if (i < nkb) {
-      volatile uint32_t late = 0;
-      for (int j = i - NS; j < i; ++j) mbar_wait(smem_u32(&ctl->full[j % NS]), (j / NS) & 1, &late, g.wait_budget_ns);
-    }
+    loads_land(&ctl->full[0], NS, static_cast<uint32_t>(min(i, nkb)), g.wait_budget_ns);
   } else if (warp == 1) {
     constexpr uint32_t idesc = make_idesc_bf16(128, TN);
     const uint64_t dw0 = make_smem_desc_sw128(base), dx0 = make_smem_desc_sw128(base + KPS * kWTileBytes);

@@ -33,3 +33,22 @@ def test_epilogue_warps_that_meet_at_barriers_leave_together():
         meets = "epilogue_warps_" in struct[1]
         assert f"kWarpsMeet = {'true' if meets else 'false'};" in struct[1], struct[0]
     assert not re.findall(r"epilogue_warps_sync\(\);\s*if \(\*abort_flag", fused)
+
+
+@pytest.mark.parametrize("name", ["gemm_kernel.cuh", "gemm2_kernel.cuh", "gemm_small.cu"])
+def test_a_producer_stays_until_its_loads_have_landed(name):
+    """Shared memory must not go away under a load in flight, whichever role gave up first: the last thing the
+    producer does, on every path, is to wait (bounded) for its last loads, with an abort flag of its own."""
+    text = _source(name)
+    producer = text[re.search(r"if \(warp == 0\) \{\s*uint32_t", text).start():]
+    producer = producer[:producer.index("} else if (warp == 1)")]
+    assert re.search(r"loads_land\(&ctl->full\[0\], NS, [^;]*\);\s*(if \(!ok\) loads_land\([^;]*;\s*\})?\s*$", producer), producer[-300:]
+    land = _source("gemm_kernel.cuh")
+    land = land[land.index("void loads_land"):]
+    assert "&late, budget_ns" in land[:land.index("\n}")]
+
+
+def test_a_communication_cta_that_gives_up_lets_its_loads_land():
+    fused = _source("gemm_fused.cu")
+    comm = fused[fused.index("bulk_load("):]
+    assert re.search(r"if \(!ok\) \{\s*loads_land\(s_full, [^;]*n_loaded[^;]*;\s*return;", comm)
