@@ -13,6 +13,8 @@ import os
 import warnings
 from pathlib import Path
 
+from . import _ext_file
+
 _HERE = Path(__file__).resolve().parent
 _LIB = None
 
@@ -202,11 +204,11 @@ def ext():
     import torch  # noqa: F401  (its shared libraries must be in the process first)
 
     L = lib()
-    from . import build as _build
-    path = _build.torch_ext_path()
+    path = _ext_file.torch_ext_path()
     if path is not None and not path.exists():
         why = "MINI_NCCL_NO_BUILD=1" if os.environ.get("MINI_NCCL_NO_BUILD") == "1" else None
         if why is None:
+            from . import build as _build
             try:
                 _build.build_torch_ext()
             except (RuntimeError, OSError) as e:   # no compiler, or one that fails

@@ -29,7 +29,6 @@ CSRC = ROOT / "csrc"
 BUILD = ROOT / "build"
 LIBDIR = ROOT / "mini_nccl_b200" / "lib"
 BINDIR = ROOT / "mini_nccl_b200" / "bin"
-EXTDIR = ROOT / "mini_nccl_b200"
 
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
@@ -115,46 +114,17 @@ def lib_path() -> Path:
     return LIBDIR / "libmini_nccl.so"
 
 
-def torch_dir() -> Path | None:
-    """Where the PyTorch is that the extension can be built against: one with CUDA."""
-    import importlib.util
-
-    spec = importlib.util.find_spec("torch")
-    if spec is None or not spec.submodule_search_locations:
-        return None
-    d = Path(spec.submodule_search_locations[0])
-    return d if (d / "lib" / "libc10_cuda.so").exists() else None
-
-
-def torch_ext_path() -> Path | None:
-    """The extension's file for the installed PyTorch and this Python, or None where there is none with CUDA.  Its
-    name holds both versions and a hash of the source: a file made for another PyTorch, another Python or from
-    another source is never taken for it."""
-    import re
-    import sysconfig
-
-    at = torch_dir()
-    if at is None:
-        return None
-    version = re.search(r"^__version__ = '([^']+)'", (at / "version.py").read_text(), re.M).group(1)
-    tag = f"{version}-{sysconfig.get_config_var('SOABI')}"
-    sources = [CSRC / "torch" / "ext.cpp", *sorted((ROOT / "include").glob("*.h"))]
-    if not sources[0].exists():    # a tree without sources: what was built for these versions
-        built = sorted(EXTDIR.glob(f"_torch_ext-{tag}-*.so"))
-        return built[-1] if built else None
-    digest = hashlib.sha1(b"".join(p.read_bytes() for p in sources)).hexdigest()[:8]
-    return EXTDIR / f"_torch_ext-{tag}-{digest}.so"
-
-
 def build_torch_ext(verbose: bool = False) -> Path | None:
     """The CPython extension behind the binding's frequent calls (csrc/torch/ext.cpp), compiled against the
     installed PyTorch; None where there is none with CUDA (the same calls then go through ctypes)."""
     import sysconfig
 
-    out = torch_ext_path()
+    from . import _ext_file
+
+    out = _ext_file.torch_ext_path()
     if out is None or out.exists():
         return out
-    torch_at = torch_dir()
+    torch_at = _ext_file.torch_dir()
     BUILD.mkdir(exist_ok=True)
     # Ranks that start together and find the file missing: one compiles, the others wait for it, and nobody sees a
     # half-written file under the final name.
@@ -162,7 +132,7 @@ def build_torch_ext(verbose: bool = False) -> Path | None:
         fcntl.flock(lock, fcntl.LOCK_EX)
         if out.exists():
             return out
-        part = out.with_suffix(f".{os.getpid()}.part")
+        part = out.with_name(f"{out.name}.{os.getpid()}.part")
         cmd = ["g++", "-std=c++17", "-O2", "-fPIC", "-fvisibility=hidden", "-shared", *_common_includes(),
                "-isystem", str(torch_at / "include"), "-isystem", str(torch_at / "include" / "torch" / "csrc" / "api" / "include"),
                "-I", sysconfig.get_paths()["include"], str(CSRC / "torch" / "ext.cpp"), "-o", str(part), "-L", str(torch_at / "lib"),

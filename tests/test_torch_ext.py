@@ -26,7 +26,8 @@ def test_pytorch_without_cuda_uses_ctypes(free_port):
     code = """
 import sys, torch
 import mini_nccl_b200.build as b
-b.torch_dir = lambda: None
+from mini_nccl_b200 import _ext_file
+_ext_file.torch_dir = lambda: None
 assert b.build_torch_ext() is None
 import mini_nccl_b200 as mn
 from mini_nccl_b200 import _lib
@@ -61,11 +62,11 @@ def test_no_build_is_honoured():
     _run("""
 import warnings
 import mini_nccl_b200.build as b
-from mini_nccl_b200 import _lib
+from mini_nccl_b200 import _ext_file, _lib
 def never(*a, **k): raise AssertionError("built although MINI_NCCL_NO_BUILD=1")
 b.build_torch_ext = never
 _lib.lib()
-b.EXTDIR = b.EXTDIR / "nowhere"             # the extension's file is missing
+_ext_file.DIR = _ext_file.DIR / "nowhere"   # the extension's file is missing
 with warnings.catch_warnings(record=True) as w:
     warnings.simplefilter("always")
     assert type(_lib.ext()).__name__ == "Calls"
@@ -78,8 +79,8 @@ def test_without_a_compiler_the_calls_go_through_ctypes(tmp_path):
 import os, warnings, torch
 from pathlib import Path
 import mini_nccl_b200.build as b
-from mini_nccl_b200 import _lib
-b.EXTDIR = b.BUILD = Path(%r)
+from mini_nccl_b200 import _ext_file, _lib
+_ext_file.DIR = b.BUILD = Path(%r)
 _lib.lib()
 os.environ["PATH"] = ""                     # no g++
 with warnings.catch_warnings(record=True) as w:
@@ -91,27 +92,26 @@ assert any("g++" in str(x.message) for x in w)
 
 def test_the_file_is_that_of_this_pytorch_python_and_source(tmp_path):
     _run("""
-import sys, sysconfig, torch
+import importlib.machinery, torch
 from pathlib import Path
-import mini_nccl_b200.build as b
-from mini_nccl_b200 import _lib
-path = b.torch_ext_path()
-assert torch.__version__ in path.name and sysconfig.get_config_var("SOABI") in path.name
+from mini_nccl_b200 import _ext_file as f, _lib
+path = f.torch_ext_path()
+assert torch.__version__ in path.name and path.name.endswith(importlib.machinery.EXTENSION_SUFFIXES[0])
 assert Path(_lib.ext().__file__) == path, "the file loaded is the one of this name"
-tmp = Path(sys.argv[1]) if len(sys.argv) > 1 else Path(%r)
+tmp = Path(%r)
 other = tmp / "torch"
 (other / "lib").mkdir(parents=True)
 (other / "lib" / "libc10_cuda.so").touch()
 (other / "version.py").write_text("__version__ = '9.9.9'\\n")
-real = b.torch_dir
-b.torch_dir = lambda: other
-assert "9.9.9" in b.torch_ext_path().name and b.torch_ext_path() != path, "another PyTorch, another file"
-b.torch_dir = real
-src = b.CSRC
-b.CSRC = tmp / "csrc"
-(b.CSRC / "torch").mkdir(parents=True)
-(b.CSRC / "torch" / "ext.cpp").write_text((src / "torch" / "ext.cpp").read_text() + "// edited")
-assert b.torch_ext_path() != path, "an edited source, another file"
+real = f.torch_dir
+f.torch_dir = lambda: other
+assert "9.9.9" in f.torch_ext_path().name, "another PyTorch, another file"
+f.torch_dir = real
+src = f.CSRC
+f.CSRC = tmp / "csrc"
+(f.CSRC / "torch").mkdir(parents=True)
+(f.CSRC / "torch" / "ext.cpp").write_text((src / "torch" / "ext.cpp").read_text() + "// edited")
+assert f.torch_ext_path() not in (None, path), "an edited source, another file"
 """ % str(tmp_path))
 
 
@@ -127,8 +127,9 @@ def test_processes_that_start_together_build_it_once_and_never_see_half_a_file(t
 import sys, threading
 from pathlib import Path
 import mini_nccl_b200.build as b
-b.EXTDIR = b.BUILD = Path(%r)
-path, seen, done = b.torch_ext_path(), [], threading.Event()
+from mini_nccl_b200 import _ext_file
+_ext_file.DIR = b.BUILD = Path(%r)
+path, seen, done = _ext_file.torch_ext_path(), [], threading.Event()
 def watch():
     while not done.is_set():
         if path.exists(): seen.append(path.read_text())
@@ -145,7 +146,7 @@ assert path.read_text() == "firstsecond" and set(seen) <= {"firstsecond"}, set(s
     outs = [p.communicate(timeout=120)[0] for p in procs]
     assert [p.returncode for p in procs] == [0, 0, 0], outs
     assert (tmp_path / "runs").read_text() == "run\n"
-    assert sorted(p.suffix for p in tmp_path.glob("_torch_ext*")) == [".so"]
+    assert [p.suffix for p in tmp_path.glob("_torch_ext*")] == [".so"]
 
 
 @pytest.mark.gpu
