@@ -55,7 +55,7 @@ class _LmHeadCrossEntropy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, targets):
         V = weight.shape[0]
-        rows, w, t = _rows(x.detach()).view(-1, x.shape[-1]), _rows(weight.detach()), targets.reshape(-1).contiguous()
+        rows, w, t = _rows(x.detach()).view(-1, x.shape[-1]), _rows(weight.detach()), targets.view(-1).contiguous()
         T = rows.shape[0]
         logits = torch.empty((T, _eight(V)), dtype=x.dtype, device=x.device)
         gemm_bf16(rows, w, out=logits[:, :V])

@@ -124,3 +124,14 @@ def test_calls_that_stay_with_the_plain_operators():
     seen = []
     torch.func.vmap(lambda s: (seen.append(_native(s, w, t[0])), s)[1])(x.detach())
     assert seen == [False]
+
+
+@pytest.mark.gpu
+def test_targets_that_cannot_be_viewed_as_one_row_are_refused_by_both():
+    x, w, t = _case((4, 16), 640, 64)
+    apart = torch.cat((t, t), dim=1)[:, :16]
+    for f in (node, _reference):
+        with pytest.raises(RuntimeError, match="view"):
+            f(x, w, apart)
+    every_other = torch.stack((t, t), dim=-1)[..., 0]            # strided, but one row all the same
+    assert torch.equal(node(x, w, every_other), node(x, w, t))
