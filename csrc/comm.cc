@@ -965,7 +965,7 @@ void Comm::solo_all_reduce(const void* send, DType send_t, void* recv, DType rec
   if ((host_in || host_out) && !in_place) {
     const size_t bytes = std::max(in_bytes, out_bytes);
     const bool pipeline = cfg_.host_pipeline_min_bytes != 0 && bytes >= std::max(cfg_.host_pipeline_min_bytes, 2 * cfg_.host_chunk_bytes);
-    SoloRing* ring = pipeline ? solo_ring(stream) : nullptr;
+    SoloRing* ring = pipeline ? solo_ring(stream, bytes) : nullptr;
     if (ring != nullptr) {
       launch_solo_host(*ring, la, send_t, recv_t, stream, host_in, host_out);
       stats_.pipelined++;
@@ -1002,9 +1002,10 @@ void Comm::SoloRing::destroy() {
   if (stage) cudaFree(stage);
   s_in = s_out = nullptr;
   stage = nullptr;
+  slot_bytes = 0;
 }
 
-void Comm::create_ring(SoloRing& r) {
+void Comm::create_ring(SoloRing& r, size_t slot_bytes) {
   AllowAllocationsWhileCapturing allow;
   const auto event = [](cudaEvent_t& e) {
     if (e == nullptr) RT_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
@@ -1018,25 +1019,36 @@ void Comm::create_ring(SoloRing& r) {
     event(r.ev_work[h]);
     event(r.ev_done[h]);
   }
-  if (r.stage == nullptr) {
-    // slots for the largest chunk, so that a ring never has to grow
-    r.slot_bytes = solo_chunk_bytes(SIZE_MAX);
-    RT_CHECK(cudaMalloc(reinterpret_cast<void**>(&r.stage), kSoloSlots * r.slot_bytes), "cudaMalloc (host staging)");
+  if (r.slot_bytes < slot_bytes) {
+    if (r.stage) {
+      // calls that run may still use it; graphs do not (they hold rings of their own)
+      RT_CHECK(cudaEventSynchronize(r.ev_last), "cudaEventSynchronize");
+      RT_CHECK(cudaFree(r.stage), "cudaFree (host staging)");
+      r.stage = nullptr;
+      r.slot_bytes = 0;
+    }
+    RT_CHECK(cudaMalloc(reinterpret_cast<void**>(&r.stage), kSoloSlots * slot_bytes), "cudaMalloc (host staging)");
+    r.slot_bytes = slot_bytes;
   }
 }
 
-// The ring for a call on `stream`; null for a captured call that finds none left.
-Comm::SoloRing* Comm::solo_ring(cudaStream_t stream) {
+// The ring for a call on `stream` whose wider side has `bytes`; null for a captured call that finds none left.
+Comm::SoloRing* Comm::solo_ring(cudaStream_t stream, size_t bytes) {
+  // Slots of the chunk's size, in powers of two, so that growing messages replace the staging twice at most.
+  const size_t chunk = solo_chunk_bytes(bytes);
+  size_t slot_bytes = 65536;
+  while (slot_bytes < chunk) slot_bytes *= 2;
+  slot_bytes = std::min(slot_bytes, solo_chunk_bytes(SIZE_MAX));
   const CaptureInfo cap = capture_info(stream);
   if (!cap.active) {
-    create_ring(solo_ring_);
+    create_ring(solo_ring_, slot_bytes);
     return &solo_ring_;
   }
   // Calls of one capture on one stream run one after the other, in every replay: they share a ring.
   SoloRing* idle = nullptr;
   for (auto& r : solo_graph_rings_) {
     if (!r->in_graph->load(std::memory_order_acquire)) idle = r.get();
-    else if (r->capture_id == cap.id && r->capture_stream == stream) return r.get();
+    else if (r->capture_id == cap.id && r->capture_stream == stream && r->slot_bytes >= slot_bytes) return r.get();
   }
   if (idle == nullptr) {
     if (solo_graph_rings_.size() == kSoloGraphRings) return nullptr;
@@ -1044,7 +1056,7 @@ Comm::SoloRing* Comm::solo_ring(cudaStream_t stream) {
     idle = solo_graph_rings_.back().get();
     idle->in_graph = std::make_shared<std::atomic<bool>>(false);
   }
-  create_ring(*idle);
+  create_ring(*idle, slot_bytes);
   if (!hold_while_graph_lives(cap.graph, idle->in_graph)) return nullptr;
   idle->capture_id = cap.id;
   idle->capture_stream = stream;

@@ -94,8 +94,8 @@ class Comm {
   struct SoloRing;
   void launch_solo_host(SoloRing& ring, const LocalArgs& call, DType send_t, DType recv_t, cudaStream_t stream, bool host_in,
                         bool host_out);
-  SoloRing* solo_ring(cudaStream_t stream);
-  void create_ring(SoloRing& r);
+  SoloRing* solo_ring(cudaStream_t stream, size_t bytes);
+  void create_ring(SoloRing& r, size_t slot_bytes);
   size_t solo_chunk_bytes(size_t bytes) const;
   void ensure_pipeline();
   void ring_all_reduce(const void* send, void* recv, size_t count, DType t, RedOp op, cudaStream_t stream);
@@ -164,7 +164,7 @@ class Comm {
   // Single rank with pinned host buffers: a ring of kSoloSlots chunks of device staging, with the side streams and
   // events that walk it.  Calls that run at once share one ring, each after the one before it, whatever their
   // streams.  A captured call takes a ring of its own, because its graph replays beside them.
-  static constexpr int kSoloSlots = 8;
+  static constexpr int kSoloSlots = 4;   // 3, 6 and 8 take the same time (16 to 256 MiB, with and without a kernel)
   static constexpr size_t kSoloGraphRings = 4;   // captured calls beyond these rings take the plain kernel
   struct SoloRing {
     cudaStream_t s_in = nullptr, s_out = nullptr;

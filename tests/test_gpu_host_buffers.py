@@ -170,3 +170,33 @@ def test_rings_of_graphs_are_bounded_and_reused():
         again = None
     finally:
         comm.destroy()
+
+
+def test_staging_is_sized_for_the_message_and_grows():
+    import mini_nccl_b200 as mn
+
+    comm = mn.Communicator(1, 0)
+    try:
+        comm.all_reduce(_filled(1 << 20, 1).cuda())
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        for mib, most in ((32, 20), (200, 68), (32, 68)):            # four slots of an eighth, of 16 MB at most
+            n = (mib << 20) // 4
+            x, y = torch.randn(n).pin_memory(), torch.zeros(n).pin_memory()
+            for scale in (1.0, 2.0):
+                comm.all_reduce(x, "sum", out=y, scale=scale)
+                torch.cuda.synchronize()
+                assert torch.equal(y, x * scale)
+            assert free - torch.cuda.mem_get_info()[0] <= most << 20, mib
+        big = (160 << 20) // 4                                        # a later, larger call of one capture: a ring of its own
+        x, y, z = torch.randn(big).pin_memory(), torch.zeros(big).pin_memory(), torch.zeros(big).pin_memory()
+        g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.stream(s), torch.cuda.graph(g, stream=s):
+            comm.all_reduce(x[:big // 8], "sum", out=y[:big // 8], scale=3.0)
+            comm.all_reduce(x, "sum", out=z, scale=5.0)
+        for _ in range(2):
+            g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y[:big // 8], x[:big // 8] * 3.0) and torch.equal(z, x * 5.0)
+    finally:
+        comm.destroy()
