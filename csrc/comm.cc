@@ -964,7 +964,7 @@ void Comm::solo_all_reduce(const void* send, DType send_t, void* recv, DType rec
   const bool in_place = send == recv && send_t == recv_t && la.identity;  // nothing to do
   if ((host_in || host_out) && !in_place) {
     const size_t bytes = std::max(in_bytes, out_bytes);
-    const bool pipeline = cfg_.host_pipeline_min_bytes != 0 && bytes >= std::max(cfg_.host_pipeline_min_bytes, 2 * cfg_.host_chunk_bytes);
+    const bool pipeline = cfg_.solo_host_pipeline_min() != 0 && bytes >= cfg_.solo_host_pipeline_min();
     SoloRing* ring = pipeline ? solo_ring(stream, bytes) : nullptr;
     if (ring != nullptr) {
       launch_solo_host(*ring, la, send_t, recv_t, stream, host_in, host_out);

@@ -96,6 +96,7 @@ Config Config::from_getter(Getter get, void* ctx) {
   r.num("MINI_NCCL_STAGING_BYTES", c.staging_bytes);
   r.num("MINI_NCCL_PIPELINE_MIN_BYTES", c.pipeline_min_bytes);
   r.num("MINI_NCCL_HOST_PIPELINE_MIN_BYTES", c.host_pipeline_min_bytes);
+  c.host_pipeline_min_given = r.raw("MINI_NCCL_HOST_PIPELINE_MIN_BYTES") != nullptr;
   r.num("MINI_NCCL_HOST_CHUNK_BYTES", c.host_chunk_bytes);
   r.num("MINI_NCCL_PIPE_MIN_BYTES", c.pipe_min_bytes);
   r.num("MINI_NCCL_PIPE_CHUNK_BYTES", c.pipe_chunk_bytes);
@@ -141,6 +142,7 @@ bool Config::set_knob(const std::string& name, long long v) {
     if (name == k.name) {
       if (name == "HOST_CHUNK_BYTES" && v < (64 << 10)) return false;
       this->*(k.field) = static_cast<size_t>(v);
+      if (k.field == &Config::host_pipeline_min_bytes) host_pipeline_min_given = true;
       return true;
     }
   for (const auto& k : ints)

@@ -40,6 +40,7 @@ struct Config {
   size_t nvls_min_bytes = 0;          // MINI_NCCL_NVLS_MIN_BYTES    (0 = built-in table)
   size_t staging_bytes = 256u << 20;  // MINI_NCCL_STAGING_BYTES (per direction, per rank)
   size_t host_pipeline_min_bytes = 4u << 20;  // MINI_NCCL_HOST_PIPELINE_MIN_BYTES: pinned-host buffers of at least this size are moved by the copy engines in chunks that overlap the collective (0 = never)
+  bool host_pipeline_min_given = false;       // the value above was set by the user (environment, tuning file or knob)
   size_t host_chunk_bytes = 8u << 20;  // MINI_NCCL_HOST_CHUNK_BYTES: chunk of that pipeline
   bool auto_map = true;         // MINI_NCCL_AUTO_MAP: ordinary device buffers of the peer-to-peer two-shot AllReduce are exported over CUDA IPC when first seen and used directly once every rank has mapped them
   bool ring_sender_thread = true;  // MINI_NCCL_RING_SENDER_THREAD: the host ring sends from a second thread while the caller's thread receives and reduces (messages of 4 MB and more, providers that allow it)
@@ -72,6 +73,13 @@ struct Config {
   // Sets one numeric tuning knob by the name of its environment variable without the MINI_NCCL_
   // or a value out of range.  Only launch-tuning knobs can be set this way (not ports or timeouts).
   bool set_knob(const std::string& name, long long value);
+
+  // Where the host pipeline begins with one rank: unless the user said where, at two chunks, because below that the
+  // kernel alone is faster (4 MiB of fp32: 112 against 167 us; 16 MiB: 444 either way).  0 = never.
+  size_t solo_host_pipeline_min() const {
+    if (host_pipeline_min_given || host_pipeline_min_bytes == 0) return host_pipeline_min_bytes;
+    return host_pipeline_min_bytes > 2 * host_chunk_bytes ? host_pipeline_min_bytes : 2 * host_chunk_bytes;
+  }
   // Applies a tuning table (MINI_NCCL_TUNING_FILE; written by benchmarks/tune.py) for `nranks`:
   // text lines "<nranks> <KNOB> <value>", '#' starts a comment, nranks 0 matches every size.
   // Returns the number of knobs applied; malformed lines and unknown knobs are reported in *errors.

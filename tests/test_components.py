@@ -49,6 +49,15 @@ def test_config_pipeline_knobs(lib):
     assert c["pipeline_min_bytes"] == 1 << 20
 
 
+def test_config_host_pipeline_of_one_rank(lib):
+    """One rank starts the pipeline at two chunks, unless the user says where it starts."""
+    for env, want in (("", 16 << 20), ("MINI_NCCL_HOST_CHUNK_BYTES=1M", 4 << 20), ("MINI_NCCL_HOST_CHUNK_BYTES=16M", 32 << 20),
+                      ("MINI_NCCL_HOST_PIPELINE_MIN_BYTES=4M", 4 << 20), ("MINI_NCCL_HOST_PIPELINE_MIN_BYTES=1M", 1 << 20),
+                      ("MINI_NCCL_HOST_PIPELINE_MIN_BYTES=64M", 64 << 20), ("MINI_NCCL_HOST_PIPELINE_MIN_BYTES=0", 0)):
+        rc, c = cfg(lib, env)
+        assert rc == 0 and c["solo_host_pipeline_min"] == want, env
+
+
 @pytest.mark.parametrize("bad", ["MINI_NCCL_SLICE_SIZE=abc", "MINI_NCCL_WINDOW_SIZE=1.5x", "MINI_NCCL_NVLS_ENABLE=maybe",
                                  "MINI_NCCL_BOOTSTRAP_PORT=70000", "MINI_NCCL_SLICE_SIZE=-5"])
 def test_config_malformed_is_invalid_argument(lib, bad):

@@ -200,3 +200,20 @@ def test_staging_is_sized_for_the_message_and_grows():
         assert torch.equal(y[:big // 8], x[:big // 8] * 3.0) and torch.equal(z, x * 5.0)
     finally:
         comm.destroy()
+
+
+def test_the_pipeline_starts_where_the_user_says():
+    import mini_nccl_b200 as mn
+
+    comm = mn.Communicator(1, 0)
+    try:
+        x, y = torch.randn(1 << 20).pin_memory(), torch.zeros(1 << 20).pin_memory()   # 4 MiB
+        for knob, pipelined in ((None, 0), (1 << 20, 1), (0, 0), (8 << 20, 0)):
+            if knob is not None:
+                comm.set_knob("HOST_PIPELINE_MIN_BYTES", knob)
+            before = comm.stats()["pipelined_calls"]
+            comm.all_reduce(x, "sum", out=y.zero_(), scale=0.5)
+            torch.cuda.synchronize()
+            assert torch.equal(y, x * 0.5) and comm.stats()["pipelined_calls"] == before + pipelined, knob
+    finally:
+        comm.destroy()
