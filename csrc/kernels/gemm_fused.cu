@@ -35,6 +35,7 @@
 
 #include "kernels/comm_dev.h"
 #include "kernels/gemm2_kernel.cuh"
+#include "kernels/gemm_fused.h"
 #include "kernels/gemm_kernel.cuh"
 
 namespace mnccl {
@@ -493,9 +494,11 @@ MNCCL_EXPORT size_t mncclAgGemmBarWords(int nranks, int n_comm) { return size_t(
 // out[M/nranks, N] (rows of this rank) = sum over ranks of A_r[M, K] * B_r[N, K]^T, bf16.
 // stage_peers / flag_peers: the staging / flag buffers of EVERY rank as mapped here
 // (Communicator.peer_pointers); state: two zero-initialised device words of this rank.
+// `fused`: the fused kernel with one rank too (the test-suite's form, see gemm_fused.h).
 static int gemm_rs_launch(const void* A, const void* B, void* out, int M, int N, int K, int lda, int ldb, int ldo, int rank,
                           int nranks, void* const* stage_peers, void* const* flag_peers, uint32_t* state,
-                          const CommBinding& cb, cudaStream_t stream, const void* mc_stage = nullptr, int n_comm_ctas = 0) {
+                          const CommBinding& cb, cudaStream_t stream, const void* mc_stage = nullptr, int n_comm_ctas = 0,
+                          bool fused = false) {
   if (!A || !B || !out || !stage_peers || !flag_peers || !state) return -1;
   if (!check_common(M, N, K, rank, nranks, "GEMM->reduce-scatter")) return -2;
   if (lda == 0) lda = K;
@@ -504,7 +507,7 @@ static int gemm_rs_launch(const void* A, const void* B, void* out, int M, int N,
   // One rank owns every row and adds nothing: the tile's one rounding to bf16 is the result, so the plain
   // kernels store it where it belongs.  (Through the staging it was written, flagged, read back and
   // written again: 4096 x 4096 x 1792 took 93 us where the product alone takes 39.)
-  if (nranks == 1) return run_gemm("GEMM->reduce-scatter", A, B, out, M, N, K, lda, ldb, ldo, kOutBf16, stream);
+  if (nranks == 1 && !fused) return run_gemm("GEMM->reduce-scatter", A, B, out, M, N, K, lda, ldb, ldo, kOutBf16, stream);
   CUtensorMap ta, tb;
   std::string why;
   // CTA pairs need every rank's rows to be whole 256-row tiles (the rasterisation works on pairs of m-tiles)
@@ -617,16 +620,18 @@ MNCCL_EXPORT int mncclGemmReduceScatterBf16Switch(const void* A, const void* B, 
 // already be at rows [rank * M/nranks, ...) of its own buffer.  ready_peers / bar_peers: counter
 // and barrier words of every rank; state: two zero-initialised device words of this rank.
 // n_comm_ctas CTAs of the grid move data instead of computing (0 = default).
+// `fused`: the fused kernel with one rank too, which waits for the arrival of its own rows as for a peer's (the
+// test-suite's form, see gemm_fused.h).
 static int ag_gemm_launch(void* const* xg_peers, const void* B, void* C, int M, int N, int K, int lda, int ldb, int ldc,
                           int rank, int nranks, void* const* ready_peers, void* const* bar_peers, uint32_t* state,
-                          int n_comm_ctas, bool swiglu, const CommBinding& cb, cudaStream_t stream) {
+                          int n_comm_ctas, bool swiglu, const CommBinding& cb, cudaStream_t stream, bool fused = false) {
   if (!xg_peers || !B || !C || !state) return -1;
   if (!check_common(M, N, K, rank, nranks, "all-gather->GEMM")) return -2;
   if (swiglu && (N % 32 != 0 || (ldc != 0 && ldc % 8 != 0) || (reinterpret_cast<uintptr_t>(C) & 15u) != 0)) {
     fprintf(stderr, "[Mini-NCCL] all-gather->GEMM with SwiGLU: needs N a multiple of 32, ldc a multiple of 8 and C 16-byte aligned\n");
     return -2;
   }
-  if (nranks > 1 && (!ready_peers || !bar_peers)) return -1;
+  if ((nranks > 1 || fused) && (!ready_peers || !bar_peers)) return -1;
   if (K * 2 > kStages * kStageBytes / 4) {
     fprintf(stderr, "[Mini-NCCL] all-gather->GEMM: K too large for the row ring (max %d)\n", kStages * kStageBytes / 8);
     return -2;
@@ -635,7 +640,7 @@ static int ag_gemm_launch(void* const* xg_peers, const void* B, void* C, int M, 
   if (ldb == 0) ldb = K;
   if (ldc == 0) ldc = swiglu ? N / 2 : N;
   // one rank: its rows are all there is, nothing to gather
-  if (nranks == 1)
+  if (nranks == 1 && !fused)
     return run_gemm("all-gather->GEMM", xg_peers[0], B, C, M, N, K, lda, ldb, ldc, swiglu ? kOutSwiGlu : kOutBf16, stream);
   CUtensorMap ta, tb;
   std::string why;
@@ -695,7 +700,7 @@ static int ag_gemm_launch(void* const* xg_peers, const void* B, void* C, int M, 
   g.a_ready_mult = static_cast<uint32_t>(kAgPartsPerChunk);
   g.rows_per_chunk = kBM;
   g.a_local_first = rank * tiles_m_local;
-  g.a_local_count = tiles_m_local;
+  g.a_local_count = nranks == 1 ? 0 : tiles_m_local;
   const int tiles = all_tiles;
   int n_gemm = sms - n_comm;
   if (tiles < n_gemm) n_gemm = tiles;
@@ -781,3 +786,19 @@ MNCCL_EXPORT int mncclGemmProbeFlagWait(uint64_t budget_ns, int abort_first, uin
 }
 
 }  // extern "C"
+
+namespace mnccl {
+namespace gemm {
+
+int gemm_rs_fused_one_rank(const void* A, const void* B, void* out, int M, int N, int K, void* stage, void* flags, uint32_t* state,
+                           cudaStream_t stream) {
+  return gemm_rs_launch(A, B, out, M, N, K, 0, 0, 0, 0, 1, &stage, &flags, state, CommBinding(), stream, nullptr, 0, true);
+}
+
+int ag_gemm_fused_one_rank(void* xg, const void* B, void* C, int M, int N, int K, void* ready, void* bar, uint32_t* state, bool swiglu,
+                           cudaStream_t stream) {
+  return ag_gemm_launch(&xg, B, C, M, N, K, 0, 0, 0, 0, 1, &ready, &bar, state, 0, swiglu, CommBinding(), stream, true);
+}
+
+}  // namespace gemm
+}  // namespace mnccl

@@ -23,6 +23,9 @@
 #include "core/config.h"
 #include "core/error.h"
 #include "core/log.h"
+#ifndef MNCCL_HOST_ONLY_SELFTEST
+#include "kernels/gemm_fused.h"
+#endif
 #include "net/nic_select.h"
 #include "net/reg_cache.h"
 #include "net/request_pool.h"
@@ -110,6 +113,14 @@ MNCCL_EXPORT int mnccl_test_tuning_text(const char* text, int nranks, char* out,
 
 // Dirties the control words of the allocation-free entry point's static scratch (of THIS library's copy).
 #ifndef MNCCL_HOST_ONLY_SELFTEST  // the sanitizer self-test links no CUDA code
+MNCCL_EXPORT int mnccl_test_gemm_rs_fused(const void* A, const void* B, void* out, int M, int N, int K, void* stage, void* flags,
+                                          uint32_t* state, cudaStream_t stream) {
+  return gemm::gemm_rs_fused_one_rank(A, B, out, M, N, K, stage, flags, state, stream);
+}
+MNCCL_EXPORT int mnccl_test_ag_gemm_fused(void* xg, const void* B, void* C, int M, int N, int K, void* ready, void* bar, uint32_t* state,
+                                          int swiglu, cudaStream_t stream) {
+  return gemm::ag_gemm_fused_one_rank(xg, B, C, M, N, K, ready, bar, state, swiglu != 0, stream);
+}
 MNCCL_EXPORT int mnccl_test_noalloc_dirty(int byte) { return noalloc_dirty_control(byte); }
 #endif
 
