@@ -3,15 +3,17 @@ larger than the L2 but far below a GB, so that a capture ends by itself within a
 
   python benchmarks/profile_targets.py --target gemm        # tcgen05 GEMM, 4096 x 3584 x 4096, single-CTA tiles
   python benchmarks/profile_targets.py --target gemm_pair   # the same product on CTA pairs (cta_group::2)
-  python benchmarks/profile_targets.py --target copy        # fused cast/scale copy kernel, 256 MiB
+  python benchmarks/profile_targets.py --target copy        # one rank: copy with scale and cast, 256 MiB
   python benchmarks/profile_targets.py --target twoshot     # emulated 4-rank two-shot AllReduce, 64 MiB per rank
   python benchmarks/profile_targets.py --target oneshot     # emulated 4-rank one-shot AllReduce, 256 KiB per rank
+  python benchmarks/profile_targets.py --target gemm_small  # the kernel for small products, 16 x 14336 x 4096
   python benchmarks/profile_targets.py --target gemm_rs     # fused GEMM->reduce-scatter kernel, one rank, 4096 x 4096 x 1792
   python benchmarks/profile_targets.py --target ag_gemm     # fused all-gather->GEMM kernel with the SwiGLU epilogue, one rank, 4096 x 3584 x 4096
+  python benchmarks/profile_targets.py --target lm_loss     # cross-entropy of a language-model head, forward and backward, 2048 x 50257
   python benchmarks/profile_targets.py --target swiglu      # one-pass SwiGLU kernel, 4096 x 2 x 14336 bf16 in
   python benchmarks/profile_targets.py --target ll          # emulated 4-rank LL AllReduce, 32 KiB per rank
   python benchmarks/profile_targets.py --target pipe        # emulated 4-rank pipelined AllReduce (peer-to-peer form), 64 MiB per rank, ordinary buffers
-  python benchmarks/profile_targets.py --target noalloc     # allocation-free one-shot AllReduce over 4 buffers of 64 KiB
+  python benchmarks/profile_targets.py --target noalloc     # allocation-free AllReduce over 4 buffers of 64 KiB
 """
 from __future__ import annotations
 
@@ -32,7 +34,7 @@ def main():
     from mini_nccl_b200 import _lib
 
     ap = argparse.ArgumentParser()
-    ap.add_argument("--target", required=True, choices=["gemm", "gemm_pair", "copy", "twoshot", "oneshot", "gemm_rs", "ag_gemm", "swiglu", "ll", "pipe", "noalloc", "auto_direct"])
+    ap.add_argument("--target", required=True, choices=["gemm", "gemm_pair", "gemm_small", "lm_loss", "copy", "twoshot", "oneshot", "gemm_rs", "ag_gemm", "swiglu", "ll", "pipe", "noalloc", "auto_direct"])
     ap.add_argument("--launches", type=int, default=4)
     args = ap.parse_args()
     torch.cuda.set_device(0)
@@ -50,36 +52,54 @@ def main():
             gemm_bf16(a, b, out=c)
         torch.cuda.synchronize()
         assert gemm_status() == 0
-    elif args.target == "gemm_rs":
-        # single rank: the fused kernel's own code path (tile push into the staging slot, flags,
-        # owner-side reduction) with local memory standing in for the peers
-        from mini_nccl_b200.ops import GemmReduceScatter, gemm_status
+    elif args.target == "gemm_small":
+        from mini_nccl_b200.ops import gemm_bf16, gemm_status
 
-        comm = mn.Communicator(1, 0)
-        rs = GemmReduceScatter(comm, 4096, 4096)
-        a = torch.randn(4096, 1792, device="cuda").to(torch.bfloat16)
-        b = torch.randn(4096, 1792, device="cuda").to(torch.bfloat16)
-        for _ in range(args.launches):
-            rs(a, b)
+        a = torch.randn(16, 4096, device="cuda").to(torch.bfloat16)
+        weights = [torch.randn(14336, 4096, device="cuda").to(torch.bfloat16) for _ in range(2)]   # 117 MB each, taken in turn
+        for k in range(args.launches):
+            gemm_bf16(a, weights[k % 2])
         torch.cuda.synchronize()
         assert gemm_status() == 0
-        comm.destroy()
-    elif args.target == "ag_gemm":
-        # single rank: the kernel's own code path (rows already local, no communication CTAs) with the
-        # SwiGLU epilogue the tensor-parallel block uses: act [4096, 1792] out of a 4096 x 3584 x 4096 product
-        from mini_nccl_b200.ops import AllGatherGemm, gemm_status, interleave_gate_up
-
-        comm = mn.Communicator(1, 0)
-        ag = AllGatherGemm(comm, 4096, 4096)
-        ag.local_shard.copy_(torch.randn(4096, 4096, device="cuda").to(torch.bfloat16))
-        w = interleave_gate_up((torch.randn(1792, 4096, device="cuda") * 0.02).to(torch.bfloat16),
-                               (torch.randn(1792, 4096, device="cuda") * 0.02).to(torch.bfloat16))
-        act = torch.empty(4096, 1792, device="cuda", dtype=torch.bfloat16)
+    elif args.target in ("gemm_rs", "ag_gemm"):
+        # One rank, through the test-suite's library (the public entry points leave one rank to the plain GEMM): tile push
+        # into the staging, flags and the owner's reduction; or the producer's look at the row counters, communication
+        # CTAs without a peer, and the SwiGLU epilogue (act [4096, 1792] out of a 4096 x 3584 x 4096 product).
+        hooks = _lib.hooks_lib()
+        vp, i = C.c_void_p, C.c_int
+        hooks.mnccl_test_gemm_rs_fused.argtypes = [vp, vp, vp, i, i, i, vp, vp, vp, vp]
+        hooks.mnccl_test_ag_gemm_fused.argtypes = [vp, vp, vp, i, i, i, vp, vp, vp, i, vp]
+        hooks.mncclGemmRsStageBytes.restype = C.c_size_t
+        M, N, K = (4096, 4096, 1792) if args.target == "gemm_rs" else (4096, 3584, 4096)
+        a, b = (torch.randn(r, K, device="cuda").to(torch.bfloat16) for r in (M, N))
+        words = [torch.zeros(8192, dtype=torch.int32, device="cuda") for _ in range(3)]
+        stream = torch.cuda.current_stream().cuda_stream
+        if args.target == "gemm_rs":
+            stage = torch.zeros(hooks.mncclGemmRsStageBytes(M, N, 1), dtype=torch.uint8, device="cuda")
+            out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        else:
+            words[0][:M // 128] = 4 * args.launches            # every row has arrived, for all calls
+            out = torch.empty(M, N // 2, device="cuda", dtype=torch.bfloat16)
         for _ in range(args.launches):
-            ag(w, out=act, swiglu=True)
+            if args.target == "gemm_rs":
+                rc = hooks.mnccl_test_gemm_rs_fused(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, stage.data_ptr(),
+                                                    words[0].data_ptr(), words[1].data_ptr(), stream)
+            else:
+                rc = hooks.mnccl_test_ag_gemm_fused(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, words[0].data_ptr(),
+                                                    words[2].data_ptr(), words[1].data_ptr(), 1, stream)
+            assert rc == 0, rc
         torch.cuda.synchronize()
-        assert gemm_status() == 0
-        comm.destroy()
+        st = C.c_uint32()
+        assert hooks.mncclGemmStatus(C.byref(st)) == 0 and st.value == 0
+    elif args.target == "lm_loss":
+        from mini_nccl_b200.ops.lm_loss import _LmHeadCrossEntropy
+
+        x = (torch.randn(2048, 1024, device="cuda") * 0.5).to(torch.bfloat16).requires_grad_()
+        w = (torch.randn(50257, 1024, device="cuda") * 0.02).to(torch.bfloat16).requires_grad_()
+        t = torch.randint(0, 50257, (2048,), device="cuda")
+        for _ in range(args.launches):
+            _LmHeadCrossEntropy.apply(x, w, t).backward()      # 206 MB of logits
+        torch.cuda.synchronize()
     elif args.target == "swiglu":
         from mini_nccl_b200.ops import swiglu_bf16
 

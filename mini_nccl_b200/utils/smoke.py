@@ -54,8 +54,8 @@ def run() -> None:
                 assert np.array_equal(b.cpu().numpy(), want), f"algorithm {algo} mismatch"
     finally:
         lib.mncclEmuDestroy(world)
-    # tcgen05 GEMM on single-CTA tiles and on CTA pairs, and the two fused tensor-parallel kernels
-    # with one rank, against an fp32 matmul.
+    # tcgen05 GEMM on single-CTA tiles, on CTA pairs and as the kernel for small products, which one rank's calls of the
+    # two fused tensor-parallel operations take, against an fp32 matmul.
     from mini_nccl_b200.ops import gemm_bf16, gemm_status
     from mini_nccl_b200.ops.fused import AllGatherGemm, GemmReduceScatter
     from mini_nccl_b200.ops.gemm import set_pair_mode
@@ -80,4 +80,4 @@ def run() -> None:
         assert (got.float() - ref).abs().max().item() <= 2e-2 * ref.abs().max().item(), name + " mismatch"
     assert gemm_status() == 0
     solo.destroy()
-    print(f"smoke ok: loss={loss.item():.4f} buckets={len(ddp.buckets)} kernels=local,ll,oneshot,twoshot,gemm,gemm_pair,gemm_rs,ag_gemm")
+    print(f"smoke ok: loss={loss.item():.4f} buckets={len(ddp.buckets)} kernels=local,ll,oneshot,twoshot,gemm,gemm_pair,gemm_small")

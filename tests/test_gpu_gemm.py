@@ -87,9 +87,8 @@ def test_gemm_many_more_tiles_than_sms():
 
 
 def test_fused_kernels_single_rank():
-    # One rank: the same kernels run locally (push to the own staging slot, reduce one slot; no
-    # communication CTAs).  Checks the epilogue hooks, the epochs over repeated calls and the
-    # staging halves.
+    # One rank has nobody to exchange with: its calls run the plain GEMM.  Checks the route and the objects over
+    # repeated calls (the fused kernels themselves: test_gpu_gemm_fused.py).
     import mini_nccl_b200 as mn
     from mini_nccl_b200.ops import AllGatherGemm, GemmReduceScatter, gemm_status
 
@@ -115,8 +114,8 @@ def test_fused_kernels_single_rank():
 
 
 def test_fused_kernels_single_rank_bit_exact_against_the_host_oracle():
-    """Integer-valued operands: both fused kernels must reproduce the host restatement bit for bit
-    (the rounding of every partial tile to bf16 before it travels included)."""
+    """Integer-valued operands: one rank's calls must reproduce the host restatement of both fused operations bit
+    for bit."""
     import mini_nccl_b200 as mn
     from mini_nccl_b200.utils import verify
 
@@ -130,7 +129,7 @@ def test_fused_kernels_single_rank_bit_exact_against_the_host_oracle():
 
 @pytest.mark.parametrize("M,F,K", [(256, 128, 192), (512, 1792, 512), (384, 272, 128)])
 def test_all_gather_gemm_with_swiglu_in_the_epilogue(M, F, K):
-    """act = silu(X Wg^T) * (X Wu^T) out of ONE kernel (weights interleaved in groups of 16 rows) against a
+    """One rank's act = silu(X Wg^T) * (X Wu^T) out of ONE kernel (weights interleaved in groups of 16 rows) against a
     plain PyTorch fp32 computation; the (gate | up) matrix is never written."""
     import mini_nccl_b200 as mn
     from mini_nccl_b200.ops import AllGatherGemm, gemm_status, interleave_gate_up, split_gate_up

@@ -1,7 +1,7 @@
 """Pinned host buffers on one GPU: the reference's programs hand pinned host memory to
-ncclAllReduce (src/main.cpp:35, tests/perf_test.cpp:78-79).  From a few megabytes up the copy
-engines move such buffers in chunks (host -> device, kernel, device -> host as a pipeline);
-the result must equal a plain PyTorch fp32 computation."""
+ncclAllReduce (src/main.cpp:35, tests/perf_test.cpp:78-79).  From 16 MB up the copy engines move such
+buffers in chunks through a ring of four slots (host -> device, kernel, device -> host as a pipeline), below
+that the kernel reads and writes them itself; the result must equal a plain PyTorch fp32 computation."""
 import pytest
 
 torch = pytest.importorskip("torch")
@@ -19,7 +19,7 @@ def comm():
 
 
 def test_host_in_host_out_scaled(comm):
-    n = (5 << 20) + 777                       # 20 MB: three chunks of 8 MB, ragged tail
+    n = (5 << 20) + 777                       # 20 MB: five chunks of 4 MB and a ragged tail
     x = torch.randn(n).pin_memory()
     y = torch.zeros(n).pin_memory()
     before = comm.stats()["pipelined_calls"]
@@ -29,13 +29,15 @@ def test_host_in_host_out_scaled(comm):
     assert comm.stats()["pipelined_calls"] == before + 1
 
 
-def test_host_in_place(comm):
-    n = 3 << 20
+@pytest.mark.parametrize("n,pipelined", [(3 << 20, 0), ((10 << 20) + 3, 1)], ids=["kernel", "ring"])
+def test_host_in_place(comm, n, pipelined):
     x = torch.randn(n).pin_memory()
     ref = x.clone()
+    before = comm.stats()["pipelined_calls"]
     comm.all_reduce(x, "sum", scale=2.0)
     torch.cuda.synchronize()
     assert torch.equal(x, ref * 2.0)
+    assert comm.stats()["pipelined_calls"] == before + pipelined
 
 
 def test_host_to_device_and_back_with_cast(comm):
@@ -61,22 +63,27 @@ def test_small_host_buffer_takes_the_direct_kernel(comm):
     assert comm.stats()["pipelined_calls"] == before
 
 
-def test_host_pipeline_in_cuda_graph(comm):
-    n = 3 << 20
+@pytest.mark.parametrize("scale", [3.0, 1.0], ids=["kernel", "copy_engines_only"])
+@pytest.mark.parametrize("n,pipelined", [(3 << 20, 0), ((10 << 20) + 3, 1)], ids=["direct", "ring"])
+def test_host_pipeline_in_cuda_graph(comm, n, pipelined, scale):
     x = torch.randn(n).pin_memory()
     y = torch.zeros(n).pin_memory()
     g = torch.cuda.CUDAGraph()
     s = torch.cuda.Stream()
     s.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(s):
-        comm.all_reduce(x, "sum", out=y, scale=3.0)   # warm-up outside capture (allocates the staging)
+        comm.all_reduce(x, "sum", out=y, scale=scale)   # a warm-up outside capture
         s.synchronize()
+        before = comm.stats()["pipelined_calls"]
         with torch.cuda.graph(g, stream=s):
-            comm.all_reduce(x, "sum", out=y, scale=3.0)
-    y.zero_()
-    g.replay()
-    torch.cuda.synchronize()
-    assert torch.equal(y, x * 3.0)
+            comm.all_reduce(x, "sum", out=y, scale=scale)
+    assert comm.stats()["pipelined_calls"] == before + pipelined
+    for _ in range(2):
+        y.zero_()
+        x.neg_()                                         # a replay moves what is there now
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, x * scale)
 
 
 def _filled(n, value):

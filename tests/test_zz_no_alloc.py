@@ -3,8 +3,7 @@ and compared with the entry point that allocates its scratch (the emulated one-s
 
 Collected last on purpose (pytest orders files by name): a run that stops at the first failure
 has then already run every other test.  It shares no state with them: it must pass alone in a
-fresh process and after the whole suite, which is why it loads the library itself and makes
-two calls in a row on the same static scratch (the second one sees what the first left)."""
+fresh process and after the whole suite, which is why it loads the library itself and makes two calls in a row."""
 import ctypes as C
 
 import numpy as np
@@ -43,11 +42,11 @@ def test_no_alloc_matches_allocating_entry_point_twice_in_a_row():
     import torch
 
     L, lib = _lib()
-    assert 0 < lib.mncclNoAllocScratchBytes() <= 8 << 20, "the static scratch is meant to be modest"
+    assert 0 < lib.mncclNoAllocScratchBytes() <= 8 << 20, "the static memory is meant to be modest"
     cases = [(4, 16384, L.FLOAT32, torch.float32, L.SUM), (3, 4099, L.BFLOAT16, torch.bfloat16, L.AVG),
              (2, 777, L.INT32, torch.int32, L.MAX), (4, 32768, L.FLOAT16, torch.float16, L.SUM)]
     for n, count, code, tdt, op in cases:
-        for call in range(2):  # two calls in a row share the static scratch
+        for call in range(2):
             g = torch.Generator(device="cuda").manual_seed(1234 + call)
             if tdt == torch.int32:
                 ins = [torch.randint(-1000, 1000, (count,), generator=g, device="cuda", dtype=tdt) for _ in range(n)]
@@ -60,7 +59,7 @@ def test_no_alloc_matches_allocating_entry_point_twice_in_a_row():
             rc = lib.mncclLocalAllReduceNoAlloc(sp, rp, n, count, code, op, None)
             assert rc == 0, f"rc {rc}"
             torch.cuda.synchronize()
-            # both entry points run the same rank-ordered kernel body: the results are the same bits
+            # both entry points add in buffer order: the results are the same bits
             for r in range(n):
                 assert torch.equal(outs[r].cpu(), want[r]), (n, count, tdt, op, call, r)
             st, det = C.c_uint(7), C.c_uint(7)
@@ -74,13 +73,13 @@ def test_no_alloc_matches_allocating_entry_point_twice_in_a_row():
 
 def test_no_alloc_allocates_nothing_and_ignores_what_the_last_call_left():
     """Free device memory is the same before and after a call (the first call on the device may load the
-    kernel, so the check is on a later one), and a call does not depend on the control words the one
-    before it left behind: the scratch is dirtied with a direct copy between two calls."""
+    kernel, so the check is on a later one), and a call leaves its own outcome whatever was in the record: it is
+    dirtied with a direct copy between two calls."""
     import torch
 
     L, _ = _lib()
     # every call of this test goes through the test-suite's own copy of the library: the hook that
-    # dirties the scratch acts on that copy's static array
+    # dirties the record acts on that copy's static memory
     lib = L.hooks_lib()
     lib.mncclLocalAllReduceNoAlloc.restype = C.c_int
     lib.mncclLocalAllReduceNoAlloc.argtypes = [C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.c_int, C.c_size_t, C.c_int, C.c_int, C.c_void_p]
@@ -101,7 +100,7 @@ def test_no_alloc_allocates_nothing_and_ignores_what_the_last_call_left():
     assert rt.cudaMemGetInfo(C.byref(free1), C.byref(total)) == 0
     assert free1.value == free0.value, "the call changed the amount of free device memory"
     assert all(torch.equal(o, torch.full_like(o, 10.0)) for o in outs)
-    # leave garbage in the barrier words and the per-rank state (as an aborted call would), call again
+    # leave garbage in the outcome record, call again
     assert lib.mnccl_test_noalloc_dirty(0xA5) == 0
     for o in outs:
         o.zero_()
@@ -112,7 +111,28 @@ def test_no_alloc_allocates_nothing_and_ignores_what_the_last_call_left():
     assert lib.mncclNoAllocLastStatus(None, C.byref(st), None) == 0 and st.value == 0
 
 
-def test_no_alloc_rejects_what_exceeds_the_static_scratch():
+def test_no_alloc_calls_that_overlap_on_two_streams():
+    """Calls keep nothing between them, so calls on streams that nothing orders do not disturb one another."""
+    import torch
+
+    L, lib = _lib()
+    n, count = 4, 16384
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    ins = [[torch.randn(count, device="cuda") for _ in range(n)] for _ in streams]
+    outs = [[[torch.zeros_like(t) for t in mine] for _ in range(50)] for mine in ins]
+    torch.cuda.synchronize()
+    for it in range(50):
+        for k, s in enumerate(streams):
+            sp = (C.c_void_p * n)(*[t.data_ptr() for t in ins[k]])
+            rp = (C.c_void_p * n)(*[t.data_ptr() for t in outs[k][it]])
+            assert lib.mncclLocalAllReduceNoAlloc(sp, rp, n, count, L.FLOAT32, L.SUM, s.cuda_stream) == 0
+    torch.cuda.synchronize()
+    for k in range(2):
+        want = ((ins[k][0] + ins[k][1]) + ins[k][2]) + ins[k][3]
+        assert all(torch.equal(o, want) for call in outs[k] for o in call)
+
+
+def test_no_alloc_rejects_what_exceeds_its_limits():
     import torch
 
     L, lib = _lib()
