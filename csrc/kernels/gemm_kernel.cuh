@@ -121,12 +121,14 @@ __device__ __forceinline__ bool accumulator_wait(uint32_t bar, uint32_t parity, 
   return ok;
 }
 
-// Last step of a producer that has issued `n` loads into a ring of `stages`: the ones still in flight land (bounded),
-// whoever gave up first, before this CTA's shared memory goes away.  After a run without failures they have landed.
+// Last step of a producer that has issued `n` loads into a ring of `stages`: the ones still in flight land (all within
+// one budget), whoever gave up first, before this CTA's shared memory goes away.  The CTA's abort flag is not asked: it
+// may be set.  After a run without failures the loads have landed.
 __device__ __forceinline__ void loads_land(uint64_t* full, uint32_t stages, uint32_t n, uint64_t budget_ns) {
-  volatile uint32_t late = 0;   // its own: the CTA's abort flag may be set, which would end every wait at once
+  const uint64_t t0 = globaltimer_ns();
   for (uint32_t j = n > stages ? n - stages : 0; j < n; ++j)
-    mbar_wait(smem_u32(full + j % stages), (j / stages) & 1u, &late, budget_ns);
+    while (!mbar_try_wait(smem_u32(full + j % stages), (j / stages) & 1u))
+      if (globaltimer_ns() - t0 > budget_ns) return;
 }
 
 struct __align__(8) SharedCtl {

@@ -154,11 +154,16 @@ bool create_split_pool(SplitPool* p, bool captured) {
 class SplitLease {
  public:
   bool take(cudaStream_t stream) {
-    SplitPools& all = split_pools();
-    lock_ = std::unique_lock<std::mutex>(all.mu);
-    const int dev = current_device_slot();
-    const CaptureInfo cap = capture_info(stream);
-    return cap.active ? take_captured(all.graph[dev], cap, stream) : take_live(all.live[dev], stream);
+    try {
+      SplitPools& all = split_pools();
+      lock_ = std::unique_lock<std::mutex>(all.mu);
+      const int dev = current_device_slot();
+      const CaptureInfo cap = capture_info(stream);
+      return cap.active ? take_captured(all.graph[dev], cap, stream) : take_live(all.live[dev], stream);
+    } catch (...) {   // out of host memory, behind a C entry point: no split
+      pool_ = nullptr;
+      return false;
+    }
   }
   float* ws() const { return pool_->ws; }
   uint32_t* cnt() const { return pool_->cnt; }

@@ -38,14 +38,15 @@ def test_epilogue_warps_that_meet_at_barriers_leave_together():
 @pytest.mark.parametrize("name", ["gemm_kernel.cuh", "gemm2_kernel.cuh", "gemm_small.cu"])
 def test_a_producer_stays_until_its_loads_have_landed(name):
     """Shared memory must not go away under a load in flight, whichever role gave up first: the last thing the
-    producer does, on every path, is to wait (bounded) for its last loads, with an abort flag of its own."""
+    producer does, on every path, is to wait (bounded) for its last loads, without asking the abort flag."""
     text = _source(name)
     producer = text[re.search(r"if \(warp == 0\) \{\s*uint32_t", text).start():]
     producer = producer[:producer.index("} else if (warp == 1)")]
     assert re.search(r"loads_land\(&ctl->full\[0\], NS, [^;]*\);\s*(if \(!ok\) loads_land\([^;]*;\s*\})?\s*$", producer), producer[-300:]
     land = _source("gemm_kernel.cuh")
     land = land[land.index("void loads_land"):]
-    assert "&late, budget_ns" in land[:land.index("\n}")]
+    land = land[:land.index("\n}")]
+    assert "abort" not in land and "budget_ns) return;" in land
 
 
 def test_a_communication_cta_that_gives_up_lets_its_loads_land():
