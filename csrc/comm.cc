@@ -635,6 +635,7 @@ std::shared_ptr<Segment> Comm::find_segment(const void* ptr, size_t bytes, size_
   return nullptr;
 }
 
+// Two ranks or more (one: solo_all_reduce).
 void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType recv_t, DType wire_t, size_t count,
                   RedOp op, double scale, Algo forced, cudaStream_t stream) {
   const bool is_float = send_t == DType::Float16 || send_t == DType::Bfloat16 || send_t == DType::Float32 ||
@@ -652,41 +653,38 @@ void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType r
   pi.op = op;
   pi.forced = forced;
   size_t in_off = 0, out_off = 0;
-  std::shared_ptr<Segment> in_seg, out_seg;
-  {
-    in_seg = find_segment(send, in_bytes, &in_off);
-    out_seg = find_segment(recv, out_bytes, &out_off);
-    // A registered buffer that was freed and whose address range now belongs to another allocation: the
-    // peers' mappings point at the old memory.  Nothing can be reduced into the right place any more
-    // (and the ranks could disagree on whether the buffer still counts as registered), so the call is
-    // refused: buffers are deregistered before they are freed.
-    for (const auto* sp : {&in_seg, &out_seg}) {
-      if (*sp && (*sp)->buffer_id != 0) {
-        const void* p = sp == &in_seg ? send : recv;
-        const unsigned long long now = allocation_id(p);
-        if (now != 0 && now != (*sp)->buffer_id) {
-          stats_.stale_registrations++;
-          fail(Result::InvalidUsage, "a buffer registered with mncclCommRegister was freed and its address range allocated "
-                                     "again; call mncclCommDeregister before freeing a registered buffer");
-        }
+  const std::shared_ptr<Segment> in_seg = find_segment(send, in_bytes, &in_off);
+  const std::shared_ptr<Segment> out_seg = find_segment(recv, out_bytes, &out_off);
+  // A registered buffer that was freed and whose address range now belongs to another allocation: the
+  // peers' mappings point at the old memory.  Nothing can be reduced into the right place any more
+  // (and the ranks could disagree on whether the buffer still counts as registered), so the call is
+  // refused: buffers are deregistered before they are freed.
+  for (const auto* sp : {&in_seg, &out_seg}) {
+    if (*sp && (*sp)->buffer_id != 0) {
+      const void* p = sp == &in_seg ? send : recv;
+      const unsigned long long now = allocation_id(p);
+      if (now != 0 && now != (*sp)->buffer_id) {
+        stats_.stale_registrations++;
+        fail(Result::InvalidUsage, "a buffer registered with mncclCommRegister was freed and its address range allocated "
+                                   "again; call mncclCommDeregister before freeing a registered buffer");
       }
     }
+  }
 
-    pi.in_symmetric = in_seg && (reinterpret_cast<uintptr_t>(send) & 15u) == 0;
-    pi.out_symmetric = out_seg && (reinterpret_cast<uintptr_t>(recv) & 15u) == 0;
-    pi.in_has_mc = in_seg && in_seg->mc;
-    pi.out_has_mc = out_seg && out_seg->mc;
-    // Buffers registered through CUDA IPC have no multicast mapping.  Where the switch is
-    // available and the message is large, the pipelined NVLS path (measured 716 GB/s at 1 GiB on
-    // 8 GPUs) beats the zero-copy peer-to-peer two-shot (624 GB/s): treat them as ordinary there.
-    const bool switch_sum = (op == RedOp::Sum || op == RedOp::Avg) &&
-                            (wire_t == DType::Float32 || wire_t == DType::Float16 || wire_t == DType::Bfloat16);
-    const size_t demote_from = cfg_.pipe_min_bytes ? cfg_.pipe_min_bytes : cfg_.pipeline_min_bytes;
-    if (mode == Mode::AllReduce && caps_.nvls && size_ > 2 && switch_sum && demote_from != 0 &&
-        count * dtype_size(wire_t) >= demote_from) {
-      if (in_seg && !in_seg->mc) pi.in_symmetric = false;
-      if (out_seg && !out_seg->mc) pi.out_symmetric = false;
-    }
+  pi.in_symmetric = in_seg && (reinterpret_cast<uintptr_t>(send) & 15u) == 0;
+  pi.out_symmetric = out_seg && (reinterpret_cast<uintptr_t>(recv) & 15u) == 0;
+  pi.in_has_mc = in_seg && in_seg->mc;
+  pi.out_has_mc = out_seg && out_seg->mc;
+  // Buffers registered through CUDA IPC have no multicast mapping.  Where the switch is
+  // available and the message is large, the pipelined NVLS path (measured 716 GB/s at 1 GiB on
+  // 8 GPUs) beats the zero-copy peer-to-peer two-shot (624 GB/s): treat them as ordinary there.
+  const bool switch_sum = (op == RedOp::Sum || op == RedOp::Avg) &&
+                          (wire_t == DType::Float32 || wire_t == DType::Float16 || wire_t == DType::Bfloat16);
+  const size_t demote_from = cfg_.pipe_min_bytes ? cfg_.pipe_min_bytes : cfg_.pipeline_min_bytes;
+  if (mode == Mode::AllReduce && caps_.nvls && size_ > 2 && switch_sum && demote_from != 0 &&
+      count * dtype_size(wire_t) >= demote_from) {
+    if (in_seg && !in_seg->mc) pi.in_symmetric = false;
+    if (out_seg && !out_seg->mc) pi.out_symmetric = false;
   }
   // Kernels dereference these pointers: pageable host memory would fault.  (One driver query per
   // buffer that is not in symmetric memory; the result also decides on the host pipeline below.)
@@ -695,7 +693,7 @@ void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType r
   if (send_kind == MemKind::PlainHost || recv_kind == MemKind::PlainHost)
     fail(Result::InvalidArgument, "buffers must be device memory or pinned host memory on the GPU data plane");
   pi.host_memory = send_kind == MemKind::PinnedHost || recv_kind == MemKind::PinnedHost;
-  pi.auto_eligible = auto_shm_ != nullptr && cfg_.auto_map && mode == Mode::AllReduce && size_ > 1 && !in_seg && !out_seg &&
+  pi.auto_eligible = auto_shm_ != nullptr && cfg_.auto_map && mode == Mode::AllReduce && !in_seg && !out_seg &&
                      send_t == wire_t && recv_t == wire_t && send_kind == MemKind::Device && recv_kind == MemKind::Device;
   Plan plan = make_plan(pi, caps_, cfg_);
   if (!plan.valid) fail(Result::InvalidArgument, std::string("no kernel for this request: ") + plan.reason);
@@ -724,7 +722,7 @@ void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType r
   // every rank launches the same kernel.
   AutoDesc auto_desc{};
   bool auto_direct = false;
-  if (auto_shm_ && cfg_.auto_map && mode == Mode::AllReduce && size_ > 1 && plan.spec.algo == Algo::TwoShot && plan.copy_in &&
+  if (auto_shm_ && cfg_.auto_map && mode == Mode::AllReduce && plan.spec.algo == Algo::TwoShot && plan.copy_in &&
       plan.copy_out && !in_seg && !out_seg && send_t == wire_t && recv_t == wire_t && send_kind == MemKind::Device &&
       recv_kind == MemKind::Device && !host_pipe) {
     LaunchSpec probe = plan.spec;
@@ -745,7 +743,7 @@ void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType r
       for (int r = 0; r < size_ && r < kAutoRanks; ++r) auto_desc.mask[r] = auto_mask_[r];
     }
   }
-  if (!auto_direct && mode == Mode::AllReduce && size_ > 1 && (plan.copy_in || plan.copy_out) &&
+  if (!auto_direct && mode == Mode::AllReduce && (plan.copy_in || plan.copy_out) &&
       (plan.spec.algo == Algo::TwoShot || plan.spec.algo == Algo::Nvls || host_pipe) &&
       ((cfg_.pipeline_min_bytes != 0 && count * dtype_size(wire_t) >= cfg_.pipeline_min_bytes) || host_pipe)) {
     launch_pipelined(send, send_t, recv, recv_t, wire_t, count, op, scale, forced, stream, host_pipe && host_in,
@@ -777,7 +775,7 @@ void Comm::launch(Mode mode, const void* send, DType send_t, void* recv, DType r
     plan.spec.auto_direct = true;
     if (plan.spec.nblocks > kAutoBlocks) plan.spec.nblocks = kAutoBlocks;
   }
-  if (size_ > 1 && (plan.spec.algo == Algo::TwoShot || plan.spec.algo == Algo::Nvls)) {
+  if (plan.spec.algo == Algo::TwoShot || plan.spec.algo == Algo::Nvls) {
     const bool zc_in = !plan.copy_in && mode != Mode::AllGather;
     const bool zc_out = !plan.copy_out && mode != Mode::ReduceScatter;
     for (int r = 0; r < size_; ++r) {
@@ -854,7 +852,9 @@ void Comm::launch_pipelined(const void* send, DType send_t, void* recv, DType re
     la.scale_d = 1.0;
     la.identity = 1;
     if (!local_kernel_exists(st, dt)) fail(Result::InvalidArgument, "no copy kernel for this type combination");
-    RT_CHECK(launch_local(st, dt, la, 96, s), "copy kernel launch");  // half of the SMs' block slots stay free for the collective
+    // 96 blocks of 256 threads: as many threads as the 48 blocks of 512 that this step was measured with on several
+    // GPUs, a twelfth of what the SMs hold; the rest is the collective's.
+    RT_CHECK(launch_local(st, dt, la, 96, s), "copy kernel launch");
   };
 
   RT_CHECK(cudaEventRecord(pipe_->ev_start, stream), "cudaEventRecord");
@@ -933,12 +933,12 @@ void Comm::launch_pipelined(const void* send, DType send_t, void* recv, DType re
 
 // One rank: out = scale * in with the types converted; every operator is the identity.  Device buffers
 // take one kernel (k_local.cu).  Pinned host buffers, by size:
-//   below two pipeline chunks (16 MB)  the same kernel reads and writes host memory itself, capped at 32
-//                                      blocks: PCIe carries both directions at once from the first byte
-//                                      (4 MiB of fp32: 112 us with 32 blocks, 151 us with 148, 167 us as
-//                                      copy in, kernel, copy out)
-//   from there on                      a chunk pipeline of copy engine in (, kernel), copy engine out
-//                                      (32 MiB: 842 us either way; 256 MiB: 6.1 against 6.7 ms)
+//   below two pipeline chunks (16 MB), unless the user says otherwise (Config::solo_host_pipeline_min):
+//                      the same kernel reads and writes host memory itself, capped at 32 blocks: PCIe carries both
+//                      directions at once from the first byte (4 MiB of fp32: 114 us; with 148 blocks 151, through
+//                      the pipeline 165)
+//   from there on      a chunk pipeline of copy engine in (, kernel), copy engine out (256 MiB: 5.72 ms, by the
+//                      kernel alone 6.70; 32 MiB: 814 and 845 us)
 void Comm::solo_all_reduce(const void* send, DType send_t, void* recv, DType recv_t, DType wire_t, size_t count, RedOp op,
                            double scale, cudaStream_t stream) {
   const bool is_float = send_t == DType::Float16 || send_t == DType::Bfloat16 || send_t == DType::Float32 || send_t == DType::Float64;
@@ -978,8 +978,8 @@ void Comm::solo_all_reduce(const void* send, DType send_t, void* recv, DType rec
 
 // Chunk of the one-rank host pipeline: an eighth of the message, between half and twice the configured
 // chunk.  Small chunks shorten the first copy in and the last copy out, which nothing overlaps, but every
-// hand-over from engine to engine costs about 10 us (B200, ms: 64 MiB 1.63 / 1.61 / 1.69 with 4 / 8 / 16 MB,
-// 256 MiB 6.48 / 6.24 / 6.14).
+// hand-over from engine to engine costs about 10 us: at 64 MiB chunks of 8 MB are 1 % faster than 4 and 5 % faster than
+// 16, at 256 MiB chunks of 16 MB are 2 % faster than 8 and 6 % faster than 4.
 size_t Comm::solo_chunk_bytes(size_t bytes) const {
   const size_t c = std::min(std::max(bytes / 8, cfg_.host_chunk_bytes / 2), 2 * cfg_.host_chunk_bytes);
   return std::max<size_t>((c + 65535) & ~size_t(65535), 65536);

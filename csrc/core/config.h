@@ -39,7 +39,7 @@ struct Config {
   size_t oneshot_max_bytes = 0;       // MINI_NCCL_ONESHOT_MAX_BYTES (0 = built-in table)
   size_t nvls_min_bytes = 0;          // MINI_NCCL_NVLS_MIN_BYTES    (0 = built-in table)
   size_t staging_bytes = 256u << 20;  // MINI_NCCL_STAGING_BYTES (per direction, per rank)
-  size_t host_pipeline_min_bytes = 4u << 20;  // MINI_NCCL_HOST_PIPELINE_MIN_BYTES: pinned-host buffers of at least this size are moved by the copy engines in chunks that overlap the collective (0 = never)
+  size_t host_pipeline_min_bytes = 4u << 20;  // MINI_NCCL_HOST_PIPELINE_MIN_BYTES: pinned-host buffers of at least this size are moved by the copy engines in chunks that overlap the collective (0 = never); one rank: solo_host_pipeline_min()
   bool host_pipeline_min_given = false;       // the value above was set by the user (environment, tuning file or knob)
   size_t host_chunk_bytes = 8u << 20;  // MINI_NCCL_HOST_CHUNK_BYTES: chunk of that pipeline
   bool auto_map = true;         // MINI_NCCL_AUTO_MAP: ordinary device buffers of the peer-to-peer two-shot AllReduce are exported over CUDA IPC when first seen and used directly once every rank has mapped them
@@ -75,7 +75,8 @@ struct Config {
   bool set_knob(const std::string& name, long long value);
 
   // Where the host pipeline begins with one rank: unless the user said where, at two chunks, because below that the
-  // kernel alone is faster (4 MiB of fp32: 112 against 167 us; 16 MiB: 444 either way).  0 = never.
+  // kernel alone is faster (fp32, us, kernel against pipeline: 4 MiB 114 / 165, 16 MiB 428 / 441, 32 MiB 845 / 814).
+  // 0 = never.
   size_t solo_host_pipeline_min() const {
     if (host_pipeline_min_given || host_pipeline_min_bytes == 0) return host_pipeline_min_bytes;
     return host_pipeline_min_bytes > 2 * host_chunk_bytes ? host_pipeline_min_bytes : 2 * host_chunk_bytes;
