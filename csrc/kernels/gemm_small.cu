@@ -90,9 +90,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
   const int kb0 = slice * g.kb_per_slice;
   const int nkb = min(num_kb, kb0 + g.kb_per_slice) - kb0;  // at least 1: the plan leaves no slice empty
 
-  // The producer and the MMA warp walk their loops as whole warps and one elected lane issues: stage
-  // addresses and descriptors then stay in uniform registers.  With the loops inside `if (lane == 0)` every
-  // MMA and every load paid for moving its operands over: 0.27 us per k-block, now 0.1x (see below).
+  // The producer and the MMA warp walk their loops as whole warps and one elected lane issues (why: mbar_wait_warp
+  // in sm100_ptx.cuh; 0.27 us per k-block of four small MMAs and two loads, now 0.16).
   const bool leader = elect_one();
   auto load = [&](int i, uint32_t s) {  // k-block i of this slice into stage s; the barrier counts both tiles' bytes
     const uint32_t full = smem_u32(&ctl->full[0]) + s * 8u, dst = base + s * kStage;

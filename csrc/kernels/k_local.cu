@@ -2,15 +2,13 @@
 // copy-out step of the chunk pipeline.
 //
 // Bound by DRAM: every byte is read once and written once, nothing else happens.  What the copy rate
-// depends on is how much is in flight and in which order the blocks walk memory (B200, fp32, 256 MiB):
-//   grid-stride loop, 4 blocks of 512 per SM, 16-byte accesses          87.1 us   (before)
-//   the same with 32-byte accesses                                      85.5 us
-//   one block per tile, 16-byte accesses                                84.1 us
-//   one block per tile, 32-byte accesses (this kernel)                  82.0 us   = 6.54 TB/s
-// The hardware's block scheduler keeps the tiles that are in flight close together, which the grid-stride
-// loop does not.  A unit is what gives the wider of the two types 32 bytes (ld / st .v8.b32), so a cast
-// moves 16 + 32 bytes per unit: 13.1 M elements bf16 -> fp32 in 15.1 us, before 20 us with 8 + 16.
-// 16-byte (or no) alignment takes the narrow form.
+// depends on is how much is in flight and in which order the blocks walk memory (B200, 256 MiB of fp32, per call
+// among others): a grid-stride loop of 4 blocks of 512 threads per SM with 16-byte accesses took 91.4 us, one block
+// per tile with 32-byte accesses, this kernel, takes 81.9 = 6.55 TB/s.  In a run of the steps one by one, 32-byte accesses
+// gave 2 %, a block per tile with 16-byte accesses 3.5 %, both together 6 %.  The hardware's block scheduler keeps the
+// tiles that are in flight close together, which the grid-stride loop does not.  A unit is what gives the wider
+// of the two types 32 bytes (ld / st .v8.b32), so a cast moves 16 + 32 bytes per unit: 13.1 M elements bf16 -> fp32 in
+// 14.5 us, before 22.6 with 8 + 16.  16-byte (or no) alignment takes the narrow form.
 #include <type_traits>
 
 #include "kernels/dev_prims.cuh"
@@ -158,7 +156,7 @@ template <typename InT, typename OutT>
 cudaError_t fire_local(const LocalArgs& a, int max_blocks, cudaStream_t stream) {
   constexpr int E = kUnitElems<InT, OutT>;
   // two units per thread in flight for a plain copy; a cast has half the bytes on one side and takes four
-  // (bf16 -> fp32, 13.1 M elements: 15.4 us with two, 15.1 us with four, 15.7 us with one)
+  // (bf16 -> fp32, 13.1 M elements: two take 2 % longer than four, one 4 %)
   constexpr int U = std::is_same<InT, OutT>::value ? 2 : 4;
   constexpr uintptr_t in_mask = E * sizeof(typename Elem<InT>::Raw) - 1, out_mask = E * sizeof(typename Elem<OutT>::Raw) - 1;
   const bool wide = (reinterpret_cast<uintptr_t>(a.send) & in_mask) == 0 && (reinterpret_cast<uintptr_t>(a.recv) & out_mask) == 0;

@@ -4,8 +4,8 @@
 // 16 bytes of every buffer, adds them in buffer order and stores the result to every destination.  At
 // these sizes (at most 4 x 64 KiB in and out) the call is launch latency: one ordinary launch with the
 // pointers by value, no clearing of state, every load of a thread in flight before the first add.
-// 4 x 64 KiB fp32: 19.9 us per call as a cooperative launch of the inbox kernel behind four memsets, of
-// which 15 us were device time.
+// 4 x 64 KiB fp32, per call through ctypes: 17.4 us as a cooperative launch of the inbox kernel behind four
+// memsets, 8.0 now, of which 1.9 are device time.
 #include "kernels/noalloc.h"
 
 #include <cuda_runtime.h>
@@ -21,8 +21,8 @@ namespace {
 
 constexpr int kThreads = 128;  // 64 KiB: 4096 vectors, 32 blocks
 
-// Outcome of the last call on this GPU: {status, detail}.  Nothing in the kernel can fail, so a call
-// leaves zeros.
+// Outcome of the last call on this GPU: {status, detail}.  Nothing in the kernel can fail, so a call leaves zeros; kept
+// because mncclNoAllocLastStatus is part of the interface.
 static __device__ unsigned g_outcome[2];
 
 struct LocalSumParams {

@@ -37,6 +37,15 @@ void mncclGemmSetPairMode(int mode);
 /* The host-side choice for an M x N product on `ctas` CTAs, without a launch (needs no GPU). */
 void mncclGemmPlan(int M, int N, int ctas, int narrow, int* tile_n, int* pair);
 
+/* Whether an M x N x K product (out: 0 bf16, 1 fp32, 2 SwiGLU) takes the kernel for small products on `sms` SMs in
+ * automatic mode (1 / 0), and its plan: rows of A per tile, CTAs that share a tile's K, one CTA per SM (deep = 1) or
+ * two.  No launch, needs no GPU. */
+int mncclGemmSmallPlan(int M, int N, int K, int out, int sms, int* tn, int* slices, int* deep);
+
+/* Whether the CTA-pair kernel cuts its last wave along K on `pairs` CTA pairs (1 / 0): the first work item that is a
+ * slice, the slices per tile, the k-blocks per slice.  No launch, needs no GPU. */
+int mncclGemmSplitPlan(int M, int N, int K, int pairs, int* first, int* slices, int* kb_per_slice);
+
 /* The tiles worker `worker` of `n_workers` (CTAs, or CTA pairs with pair = 1) visits, in the kernels'
  * own order, as (tm, tn) in 128-row tiles; host arithmetic only.  Returns the number of tiles. */
 int mncclGemmTileOrder(int M, int N, int bn, int group_m, int rotate, int pair, int n_workers, int worker, int* out_tm,
