@@ -209,6 +209,28 @@ def test_staging_is_sized_for_the_message_and_grows():
         comm.destroy()
 
 
+def test_an_idle_ring_grows_inside_a_capture():
+    """A ring that a destroyed graph gave back may be too small for the next capture: it grows there."""
+    import mini_nccl_b200 as mn
+
+    comm = mn.Communicator(1, 0)
+    try:
+        before = comm.stats()["pipelined_calls"]
+        for mib in (20, 160, 20):
+            x, y = torch.randn(mib << 18).pin_memory(), torch.zeros(mib << 18).pin_memory()
+            g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+            with torch.cuda.stream(s), torch.cuda.graph(g, stream=s):
+                comm.all_reduce(x, "sum", out=y, scale=2.0)
+            for _ in range(2):
+                g.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(y, x * 2.0), mib
+            del g
+        assert comm.stats()["pipelined_calls"] == before + 3
+    finally:
+        comm.destroy()
+
+
 def test_the_pipeline_starts_where_the_user_says():
     import mini_nccl_b200 as mn
 
